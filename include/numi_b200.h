@@ -1344,10 +1344,10 @@ enum MRBatchOrderC {
     MR_BATCH_ORDER_ROUND_ROBIN = 1u
 };
 
-/* FUSED: one kernel runs every item (register budget of the most demanding
- * world).  PER_FAMILY: one persistent launch per device-code family --
- * articulated and free-body -- running concurrently, each at its own
- * kernel's register budget and occupancy. */
+/* FUSED: one persistent launch runs every item (all worlds articulated).
+ * PER_FAMILY: one per device-code family -- articulated, an environment per
+ * warp, and free-body, an environment per CTA -- running concurrently, each
+ * at its own kernel's register budget and occupancy. */
 enum MRBatchLaunchModeC {
     MR_BATCH_LAUNCH_FUSED = 0u,
     MR_BATCH_LAUNCH_PER_FAMILY = 1u
@@ -1356,7 +1356,7 @@ enum MRBatchLaunchModeC {
 typedef struct MRBatchLaunchShapeC {
     uint32_t worlds;
     uint32_t items;                  /* environments over all rollouts */
-    uint32_t warps_per_block;        /* fused / articulated launch */
+    uint32_t warps_per_block;        /* articulated launch */
     uint32_t blocks;                 /* persistent grid: SMs x resident CTAs */
     uint32_t resident_warps_per_sm;
     uint32_t shared_bytes_per_warp;
@@ -1364,7 +1364,7 @@ typedef struct MRBatchLaunchShapeC {
     uint32_t tuned;                  /* 1 after mr_batch_tune */
     float tuned_step_milliseconds;   /* the tuner's best time of one control step */
     uint32_t mode;                   /* MRBatchLaunchModeC */
-    uint32_t scene_blocks;           /* PER_FAMILY: the free-body launch's grid (one warp per CTA) */
+    uint32_t scene_blocks;           /* PER_FAMILY: the free-body launch's grid (one environment per CTA) */
     uint32_t scene_resident_warps_per_sm;
 } MRBatchLaunchShapeC;
 

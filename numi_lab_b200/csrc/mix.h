@@ -1,6 +1,7 @@
 // Heterogeneous batch: several worlds (articulated chains and trees, free-
-// body piles of any body count) advanced by ONE persistent launch per
-// horizon of control steps.  Every resident warp repeatedly claims the next
+// body piles of any body count) advanced by ONE persistent launch per device-
+// code family and horizon of control steps.  Every resident warp (articulated)
+// or CTA (free bodies) repeatedly claims the next
 // work item from a device queue (an atomic counter over a claim-ordered
 // item list) and advances that environment of that world through the
 // horizon with the world's own device code path, until the queue is empty.
@@ -41,22 +42,23 @@ constexpr int kMixMaxWorlds = 256;
 // Shared memory one warp needs for an articulated layout (floats): the
 // layout copy plus its sections.
 int mix_articulated_warp_floats(const WarpLayout& layout);
-// ... and for a free-body world.
-int mix_scene_warp_floats();
+// ... and one CTA for a free-body world.
+int mix_scene_block_floats();
 
-// Kernel families: the fused kernel runs every item; the per-family
-// kernels run one family's items at that family's own register budget.
+// Kernel families, one persistent launch each: the articulated kernel runs
+// one environment per warp, the free-body kernels one per CTA.
 // kMixFamilySceneConvex is the free-body kernel with the support-mapped
 // (GJK / EPA) narrowphase, for batches with such pairs.
-enum MixFamily : int { kMixFamilyFused = 0, kMixFamilyArticulated = 1, kMixFamilyScene = 2, kMixFamilySceneConvex = 3 };
+enum MixFamily : int { kMixFamilyArticulated = 0, kMixFamilyScene = 1, kMixFamilySceneConvex = 2 };
 
 cudaError_t configure_mix_kernel(int family, size_t max_dynamic_smem);
 cudaError_t mix_occupancy(int family, int warps_per_block, size_t smem_per_block, int* blocks_per_sm);
 // `steps` control steps of every item: `worlds` (device) holds the
 // descriptors [steps][world_count], `items` (device) the claim order,
 // `next_item` (device) a counter that must be zero at launch.  A claimed
-// environment runs all its steps before the warp claims the next one.
-// The scene family runs one warp per CTA.
+// environment runs all its steps before the next one is claimed.  The
+// free-body families run CTAs of kSceneMaxWarps warps and take their shared
+// memory per CTA (warps_per_block 1).
 cudaError_t launch_mix_horizon(int family, const MixWorld* worlds, int world_count, int steps, const std::uint32_t* items,
                                int item_count, unsigned* next_item, int warps_per_block, int smem_floats_per_warp, int grid,
                                cudaStream_t stream);
@@ -64,9 +66,8 @@ cudaError_t launch_mix_horizon(int family, const MixWorld* worlds, int world_cou
 // The free-body family kernels (scene_step.cu); `convex`: the instance with
 // the support-mapped narrowphase.
 cudaError_t configure_mix_scene_kernel(bool convex, size_t max_dynamic_smem);
-cudaError_t mix_scene_occupancy(bool convex, int warps_per_block, size_t smem_per_block, int* blocks_per_sm);
+cudaError_t mix_scene_occupancy(bool convex, size_t smem_per_block, int* blocks_per_sm);
 cudaError_t launch_mix_scene(bool convex, const MixWorld* worlds, int world_count, int steps, const std::uint32_t* items,
-                             int item_count, unsigned* next_item, int warps_per_block, int smem_floats_per_warp, int grid,
-                             cudaStream_t stream);
+                             int item_count, unsigned* next_item, size_t smem_per_block, int grid, cudaStream_t stream);
 
 }  // namespace numi

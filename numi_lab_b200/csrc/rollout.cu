@@ -425,7 +425,7 @@ struct MRTaskRolloutHandle {
     numi::SceneModel smodel{};
     DeviceBuffer<numi::SceneModel> d_smodel;
     DeviceBuffer<std::uint32_t> d_mcount;
-    DeviceBuffer<float> d_workspace;    // scene substep tables, contacts, narrowphase scratch
+    DeviceBuffer<float> d_workspace;    // scene substep tables and contact rows
     // Scene worlds: island index per body on each control step's final
     // substep ([env][kSceneMaxBodies]), written while enabled.
     DeviceBuffer<std::uint8_t> d_island_labels;
@@ -570,6 +570,7 @@ struct MRTaskRolloutHandle {
             p.velocity_iterations = static_cast<int>(config.velocity_iterations);
             p.final_velocity_iterations = static_cast<int>(config.final_velocity_iterations);
             p.support_mapped = smodel.support_mapped;
+            p.bodies = smodel.nb;
             p.island_labels = island_labels ? d_island_labels.ptr : nullptr;
             return w;
         }
@@ -665,6 +666,7 @@ struct MRTaskRolloutHandle {
                 p.final_velocity_iterations = static_cast<int>(config.final_velocity_iterations);
                 p.q_comp = precision == MR_PRECISION_COMPENSATED ? d_qcomp.ptr : nullptr;
                 p.support_mapped = smodel.support_mapped;
+                p.bodies = smodel.nb;
                 p.island_labels = island_labels ? d_island_labels.ptr : nullptr;
                 p.audit = audit ? d_audit.ptr : nullptr;
                 check(numi::launch_scene_step(p, s), "scene step launch");
@@ -2203,19 +2205,21 @@ struct MRBatchHandle {
     int sms = 0;
     cudaStream_t stream = nullptr, side = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr, ev_fork = nullptr, ev_join = nullptr, ev_a = nullptr, ev_b = nullptr;
-    // Shared memory per warp (floats) and resident CTAs per SM of each
-    // kernel family (numi::MixFamily: fused, articulated, scene).
-    int smem_floats[3] = {0, 0, 0};
-    int blocks_per_sm[3] = {0, 0, 0};
-    int warps_per_block = 2;            // fused and articulated kernels; the scene kernel runs one warp per CTA
+    // Shared memory per warp (articulated) or CTA (free bodies), in floats,
+    // and resident CTAs per SM of each kernel family.
+    static constexpr int kFamilies = 2;  // numi::kMixFamilyArticulated, numi::kMixFamilyScene
+    int smem_floats[kFamilies] = {0, 0};
+    int blocks_per_sm[kFamilies] = {0, 0};
+    int warps_per_block = 2;            // articulated kernel; the free-body kernel's CTA advances one environment
+    // One launch when all worlds are articulated, else one per family.
     std::uint32_t mode = MR_BATCH_LAUNCH_FUSED;
     std::uint32_t order = MR_BATCH_ORDER_LONGEST_FIRST;
     bool tuned = false;
     float tuned_step_ms = 0.0f;
     std::vector<float> cost;            // per world: latency of one item (ms), the claim-order key
-    // Claim orders: every item (fused) and each family's items.
-    std::vector<std::uint32_t> items[3];
-    DeviceBuffer<std::uint32_t> d_items[3];
+    // Each family's claim order.
+    std::vector<std::uint32_t> items[kFamilies];
+    DeviceBuffer<std::uint32_t> d_items[kFamilies];
     DeviceBuffer<numi::MixWorld> d_worlds;  // [steps][worlds] of the cached advance
     DeviceBuffer<unsigned> d_next;          // one queue counter per family
     PinnedBuffer<numi::MixWorld> h_worlds;
@@ -2232,16 +2236,16 @@ struct MRBatchHandle {
     }
 
     // Some free-body world has support-mapped (GJK / EPA) pairs: its family
-    // runs the kernel instance with that narrowphase, and only per family.
+    // runs the kernel instance with that narrowphase.
     bool convex = false;
     int kernel_of(int family) const { return family == numi::kMixFamilyScene && convex ? numi::kMixFamilySceneConvex : family; }
     int wpb(int family) const { return family == numi::kMixFamilyScene ? 1 : warps_per_block; }
     int grid(int family) const { return std::max(1, blocks_per_sm[family]) * sms; }
-    std::uint32_t item_count() const { return static_cast<std::uint32_t>(items[numi::kMixFamilyFused].size()); }
+    std::uint32_t item_count() const { return static_cast<std::uint32_t>(items[0].size() + items[1].size()); }
     bool is_scene(std::uint32_t w) const { return worlds[w]->scene; }
 
     void plan_launch() {
-        for (int f = 0; f < 3; ++f) {
+        for (int f = 0; f < kFamilies; ++f) {
             blocks_per_sm[f] = 0;
             if (!smem_floats[f]) continue;
             const size_t smem = static_cast<size_t>(smem_floats[f]) * sizeof(float) * wpb(f);
@@ -2258,9 +2262,7 @@ struct MRBatchHandle {
         for (std::uint32_t w = 0; w < worlds.size(); ++w) world_order[w] = w;
         std::stable_sort(world_order.begin(), world_order.end(), [&](std::uint32_t a, std::uint32_t b) { return cost[a] > cost[b]; });
         auto push = [&](std::uint32_t w, std::uint32_t e) {
-            const std::uint32_t code = (w << numi::kMixWorldShift) | e;
-            items[numi::kMixFamilyFused].push_back(code);
-            items[is_scene(w) ? numi::kMixFamilyScene : numi::kMixFamilyArticulated].push_back(code);
+            items[is_scene(w) ? numi::kMixFamilyScene : numi::kMixFamilyArticulated].push_back((w << numi::kMixWorldShift) | e);
         };
         if (order == MR_BATCH_ORDER_LONGEST_FIRST) {
             for (std::uint32_t w : world_order)
@@ -2272,7 +2274,7 @@ struct MRBatchHandle {
                 for (std::uint32_t w : world_order)
                     if (e < worlds[w]->envs) push(w, e);
         }
-        for (int f = 0; f < 3; ++f) {
+        for (int f = 0; f < kFamilies; ++f) {
             d_items[f].resize(items[f].size());
             if (!items[f].empty())
                 check(cudaMemcpy(d_items[f].ptr, items[f].data(), items[f].size() * sizeof(std::uint32_t), cudaMemcpyHostToDevice),
@@ -2292,23 +2294,19 @@ struct MRBatchHandle {
               "batch horizon launch");
     }
 
-    // Enqueues `steps` control steps of every item on `s`: one fused launch,
-    // or one launch per family (the scene family on the side stream).
+    // Enqueues `steps` control steps of every item on `s`: one launch per
+    // family (with both, the free-body family on the side stream).
     void enqueue(std::uint32_t steps, cudaStream_t s) {
-        check(cudaMemsetAsync(d_next.ptr, 0, 3 * sizeof(unsigned), s), "batch queue reset");
-        if (mode == MR_BATCH_LAUNCH_FUSED) {
-            launch(numi::kMixFamilyFused, steps, d_items[0].ptr, static_cast<int>(items[0].size()), s);
-            return;
-        }
+        check(cudaMemsetAsync(d_next.ptr, 0, kFamilies * sizeof(unsigned), s), "batch queue reset");
         const bool art = !items[numi::kMixFamilyArticulated].empty(), scn = !items[numi::kMixFamilyScene].empty();
         if (art && scn) {
             check(cudaEventRecord(ev_fork, s), "event");
             check(cudaStreamWaitEvent(side, ev_fork, 0), "stream wait");
         }
         if (art)
-            launch(numi::kMixFamilyArticulated, steps, d_items[1].ptr, static_cast<int>(items[1].size()), s);
+            launch(numi::kMixFamilyArticulated, steps, d_items[0].ptr, static_cast<int>(items[0].size()), s);
         if (scn)
-            launch(numi::kMixFamilyScene, steps, d_items[2].ptr, static_cast<int>(items[2].size()), art ? side : s);
+            launch(numi::kMixFamilyScene, steps, d_items[1].ptr, static_cast<int>(items[1].size()), art ? side : s);
         if (art && scn) {
             check(cudaEventRecord(ev_join, side), "event");
             check(cudaStreamWaitEvent(s, ev_join, 0), "stream wait");
@@ -2333,7 +2331,7 @@ struct MRBatchHandle {
         if (desc.size() == cached.size() && std::memcmp(desc.data(), cached.data(), desc.size() * sizeof(numi::MixWorld)) == 0) return;
         drop_graph();
         d_worlds.resize(desc.size());
-        d_next.resize(3);
+        d_next.resize(kFamilies);
         h_worlds.resize(desc.size());
         std::memcpy(h_worlds.ptr, desc.data(), desc.size() * sizeof(numi::MixWorld));
         check(cudaMemcpyAsync(d_worlds.ptr, h_worlds.ptr, desc.size() * sizeof(numi::MixWorld), cudaMemcpyHostToDevice, stream),
@@ -2420,8 +2418,8 @@ struct MRBatchHandle {
 
     // Autotuner: calibrates each world's item latency (its environments
     // alone, one control step, in its family's kernel), orders the queues by
-    // it, then times the whole batch for every (launch mode, warps per CTA,
-    // claim order) candidate and keeps the fastest.  The worlds' state is
+    // it, then times the whole batch for every (claim order, articulated warps
+    // per CTA) candidate and keeps the fastest.  The worlds' state is
     // put back afterwards.
     void tune(std::uint32_t steps, const float* const* actions) {
         Snapshot snap;
@@ -2436,7 +2434,7 @@ struct MRBatchHandle {
             check(cudaMemcpy(d_own.ptr, own.data(), own.size() * sizeof(std::uint32_t), cudaMemcpyHostToDevice), "tuner items");
             const int family = is_scene(w) ? numi::kMixFamilyScene : numi::kMixFamilyArticulated;
             const float ms = best_ms(2, [&] {
-                check(cudaMemsetAsync(d_next.ptr, 0, 3 * sizeof(unsigned), stream), "batch queue reset");
+                check(cudaMemsetAsync(d_next.ptr, 0, kFamilies * sizeof(unsigned), stream), "batch queue reset");
                 launch(family, 1, d_own.ptr, static_cast<int>(own.size()), stream);
             });
             const double slots = static_cast<double>(grid(family)) * wpb(family);
@@ -2444,31 +2442,26 @@ struct MRBatchHandle {
         }
         float best = 1e30f;
         int best_wpb = warps_per_block;
-        std::uint32_t best_order = order, best_mode = mode;
-        for (const std::uint32_t md : {std::uint32_t(MR_BATCH_LAUNCH_FUSED), std::uint32_t(MR_BATCH_LAUNCH_PER_FAMILY)})
-            for (const std::uint32_t ord : {std::uint32_t(MR_BATCH_ORDER_LONGEST_FIRST), std::uint32_t(MR_BATCH_ORDER_ROUND_ROBIN)})
-                for (const int wp : {1, 2, 4}) {
-                    if (convex && md == MR_BATCH_LAUNCH_FUSED) continue;
-                    mode = md;
-                    order = ord;
-                    warps_per_block = wp;
-                    try {
-                        plan_launch();
-                    } catch (const std::exception&) {
-                        continue;
-                    }
-                    order_items();
-                    const float ms = best_ms(2, [&] { enqueue(steps, stream); }) / static_cast<float>(steps);
-                    if (ms < best) {
-                        best = ms;
-                        best_wpb = wp;
-                        best_order = ord;
-                        best_mode = md;
-                    }
+        std::uint32_t best_order = order;
+        for (const std::uint32_t ord : {std::uint32_t(MR_BATCH_ORDER_LONGEST_FIRST), std::uint32_t(MR_BATCH_ORDER_ROUND_ROBIN)})
+            for (const int wp : {1, 2, 4}) {
+                order = ord;
+                warps_per_block = wp;
+                try {
+                    plan_launch();
+                } catch (const std::exception&) {
+                    continue;
                 }
+                order_items();
+                const float ms = best_ms(2, [&] { enqueue(steps, stream); }) / static_cast<float>(steps);
+                if (ms < best) {
+                    best = ms;
+                    best_wpb = wp;
+                    best_order = ord;
+                }
+            }
         warps_per_block = best_wpb;
         order = best_order;
-        mode = best_mode;
         plan_launch();
         order_items();
         tuned = true;
@@ -2504,7 +2497,7 @@ MR_API MRBatchHandle* mr_create_batch(MRTaskRolloutHandle* const* rollouts, size
             if (h->envs > numi::kMixEnvMask) throw std::invalid_argument("a batched rollout holds at most 2^24 - 1 environments");
             for (size_t j = 0; j < i; ++j)
                 if (rollouts[j] == h) throw std::invalid_argument("a rollout appears twice in the batch");
-            if (h->scene) floats_scene = numi::mix_scene_warp_floats();
+            if (h->scene) floats_scene = numi::mix_scene_block_floats();
             else floats_art = std::max(floats_art, numi::mix_articulated_warp_floats(h->layout));
             b->worlds.push_back(h);
             // First estimate of an item's latency (ms), replaced by the tuner.
@@ -2514,14 +2507,13 @@ MR_API MRBatchHandle* mr_create_batch(MRTaskRolloutHandle* const* rollouts, size
         auto round4 = [](int x) { return (x + 3) & ~3; };
         b->smem_floats[numi::kMixFamilyArticulated] = floats_art ? round4(floats_art) : 0;
         b->smem_floats[numi::kMixFamilyScene] = floats_scene ? round4(floats_scene) : 0;
-        b->smem_floats[numi::kMixFamilyFused] = round4(std::max(floats_art, floats_scene));
-        for (int f = 0; f < 3; ++f) {
+        for (int f = 0; f < MRBatchHandle::kFamilies; ++f) {
             if (!b->smem_floats[f]) continue;
-            const size_t bytes = std::min(static_cast<size_t>(b->smem_floats[f]) * sizeof(float) * 4,
+            const size_t bytes = std::min(static_cast<size_t>(b->smem_floats[f]) * sizeof(float) * (f == numi::kMixFamilyScene ? 1 : 4),
                                           static_cast<size_t>(prop.sharedMemPerBlockOptin));
             check(numi::configure_mix_kernel(b->kernel_of(f), bytes), "batch kernel attributes");
         }
-        if (b->convex) b->mode = MR_BATCH_LAUNCH_PER_FAMILY;
+        if (floats_scene) b->mode = MR_BATCH_LAUNCH_PER_FAMILY;
         for (cudaStream_t* st : {&b->stream, &b->side}) check(cudaStreamCreateWithFlags(st, cudaStreamNonBlocking), "stream");
         for (cudaEvent_t* e : {&b->ev_in, &b->ev_out, &b->ev_fork, &b->ev_join}) check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event");
         for (cudaEvent_t* e : {&b->ev_a, &b->ev_b}) check(cudaEventCreate(e), "event");
@@ -2568,14 +2560,15 @@ MR_API int mr_batch_launch_shape(const MRBatchHandle* batch, MRBatchLaunchShapeC
         *out = MRBatchLaunchShapeC{};
         out->worlds = static_cast<uint32_t>(batch->worlds.size());
         out->items = batch->item_count();
-        const int main_family = batch->mode == MR_BATCH_LAUNCH_FUSED ? numi::kMixFamilyFused : numi::kMixFamilyArticulated;
+        const int main_family = numi::kMixFamilyArticulated;
         out->warps_per_block = static_cast<uint32_t>(batch->warps_per_block);
         out->blocks = static_cast<uint32_t>(batch->grid(main_family));
         out->resident_warps_per_sm = static_cast<uint32_t>(batch->blocks_per_sm[main_family] * batch->warps_per_block);
         out->shared_bytes_per_warp = static_cast<uint32_t>(batch->smem_floats[main_family] * sizeof(float));
         out->scene_blocks = batch->mode == MR_BATCH_LAUNCH_PER_FAMILY ? static_cast<uint32_t>(batch->grid(numi::kMixFamilyScene)) : 0u;
         out->scene_resident_warps_per_sm =
-            batch->mode == MR_BATCH_LAUNCH_PER_FAMILY ? static_cast<uint32_t>(batch->blocks_per_sm[numi::kMixFamilyScene]) : 0u;
+            batch->mode == MR_BATCH_LAUNCH_PER_FAMILY
+                ? static_cast<uint32_t>(batch->blocks_per_sm[numi::kMixFamilyScene] * numi::mix_scene_warps()) : 0u;
         out->mode = batch->mode;
         out->order = batch->order;
         out->tuned = batch->tuned ? 1u : 0u;

@@ -82,12 +82,13 @@ struct SceneParams {
     std::uint32_t* status_codes;     // [item]
     std::uint32_t* active_contacts;  // [item]
     std::uint32_t* stats;
-    float* workspace;          // [slot][scene_workspace_words()]: substep tables, contacts, narrowphase scratch
+    float* workspace;          // [slot][scene_workspace_words()]: substep tables, contact rows and arrays beyond the CTA's
     std::int32_t env_count;    // items in this launch
     std::int32_t substeps;
     std::int32_t velocity_iterations;
     std::int32_t final_velocity_iterations;
     float* q_comp;             // [slot][nb][7]: compensation of the position sums (entries 0-2), or null (FP32 sums)
+    std::int32_t bodies;       // SceneModel::nb (sizes the launch's shared memory)
     std::int32_t support_mapped;  // the model has support-mapped (cylinder) pairs: SceneModel::support_mapped
     // Non-zero: the launch was enqueued for the record with this tag.  A
     // launch that finds another record behind `model` (a shared record
@@ -102,7 +103,16 @@ struct SceneParams {
     double* audit;             // [slot][kAuditWords] FP64 energy / momentum audit (audit.cuh), or null
 };
 
-size_t scene_step_smem_bytes(bool compensated = false);
+// Most warps of a CTA advancing one environment.
+constexpr int kSceneMaxWarps = 4;
+// Launch shape of the free-body kernel: warps and shared memory per CTA.
+struct SceneShape {
+    int warps;
+    size_t smem;
+};
+// ... of the batch's free-body family, for any mix of worlds.
+int mix_scene_warps();
+size_t mix_scene_smem_bytes();
 size_t scene_workspace_words();
 cudaError_t configure_scene_step_kernel();
 cudaError_t launch_scene_step(const SceneParams& p, cudaStream_t stream);

@@ -4,65 +4,49 @@
 #include "mix.h"
 #include "scene_step.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 
 namespace numi {
 namespace {
 
-// The FP32 control step of a world with support-mapped pairs, compiled once
-// out of line: the per-world kernel and the batch's free-body family both
-// call this body, so the two produce the same bits (inlined into two
-// kernels, the compiler's floating-point contractions may differ).
-__device__ __noinline__ void scene_step_convex(const SceneParams& p, float* smem, int item, int env) {
-    scene_step_item<false, true>(p, smem, item, env);
-}
-
-// At most 128 registers: 16 resident warps per SM.  More warps (96
-// registers) ran slower: their narrowphase scratch no longer fits the L1.
+// 128 registers: 16 warps per SM, i.e. four environments of four warps.  At
+// 96 registers (20 warps) the spills cost more than the warps gave: 36-body
+// piles 10.3 against 9.8 ms.
 template <bool kComp, bool kConvex>
-__global__ void __launch_bounds__(32, 16) scene_step_kernel(SceneParams p) {
+__global__ void __launch_bounds__(32 * kSceneMaxWarps, 16 / kSceneMaxWarps) scene_step_kernel(const __grid_constant__ SceneParams p) {
     extern __shared__ float4 smem4[];
     const int item = blockIdx.x;
-    if (item >= p.env_count) return;
     const int env = p.env_index != nullptr ? p.env_index[item] : item;
-    if constexpr (!kComp && kConvex)
-        scene_step_convex(p, reinterpret_cast<float*>(smem4), item, env);
-    else
-        scene_step_item<kComp, kConvex>(p, reinterpret_cast<float*>(smem4), item, env);
+    scene_step_item<kComp, kConvex>(p, reinterpret_cast<float*>(smem4), item, env);
 }
 
-// The batch's free-body family (mix_step.cu): the per-family claim loop over
-// free-body items.  It sits in this translation unit so that it and the
-// per-world kernel run one compiled copy of the out-of-line narrowphase
-// (support_mapped_contacts): a batch reproduces each world alone bit for
-// bit.  A world without support-mapped pairs runs the instance its own
-// kernel runs.
+// The batch's free-body family (mix_step.cu): the claim loop over free-body
+// items, one CTA per item.  It sits in this translation unit so that it and
+// the per-world kernel call one compiled copy of the control step: a batch
+// reproduces each world alone bit for bit.
 template <bool kConvex>
-__global__ void __launch_bounds__(32, 16) mix_scene_kernel(const MixWorld* __restrict__ worlds, int world_count, int steps,
-                                                           const std::uint32_t* __restrict__ items, int item_count,
-                                                           unsigned* next_item, int smem_floats_per_warp) {
+__global__ void __launch_bounds__(32 * kSceneMaxWarps, 16 / kSceneMaxWarps)
+    mix_scene_kernel(const MixWorld* __restrict__ worlds, int world_count, int steps, const std::uint32_t* __restrict__ items,
+                     int item_count, unsigned* next_item) {
     extern __shared__ float4 smem4[];
-    const int lane = threadIdx.x & 31;
-    float* base = reinterpret_cast<float*>(smem4) + static_cast<size_t>(threadIdx.x >> 5) * smem_floats_per_warp;
+    __shared__ unsigned next;
     for (;;) {
-        unsigned claimed = 0u;
-        if (lane == 0) claimed = atomicAdd(next_item, 1u);
-        claimed = __shfl_sync(0xffffffffu, claimed, 0);
+        if (threadIdx.x == 0) next = atomicAdd(next_item, 1u);
+        __syncthreads();
+        const unsigned claimed = next;
+        __syncthreads();
         if (claimed >= static_cast<unsigned>(item_count)) break;
         const std::uint32_t code = items[claimed];
         const int world = static_cast<int>(code >> kMixWorldShift);
         const int env = static_cast<int>(code & kMixEnvMask);
         for (int k = 0; k < steps; ++k) {
             const SceneParams& sp = worlds[static_cast<size_t>(k) * world_count + world].scene;
-            if constexpr (kConvex) {
-                if (sp.support_mapped)
-                    scene_step_convex(sp, base, env, env);
-                else
-                    scene_step_item<false, false>(sp, base, env, env);
-            } else {
-                scene_step_item<false, false>(sp, base, env, env);
-            }
-            __syncwarp();
+            if (kConvex && sp.support_mapped)
+                scene_step_item<false, true>(sp, reinterpret_cast<float*>(smem4), env, env);
+            else
+                scene_step_item<false, false>(sp, reinterpret_cast<float*>(smem4), env, env);
+            __syncthreads();
         }
     }
 }
@@ -81,15 +65,11 @@ __global__ void __launch_bounds__(32) scene_audit_kernel(SceneParams p) {
 
 }  // namespace
 
-size_t scene_step_smem_bytes(bool compensated) {
-    return static_cast<size_t>(compensated ? kSceneSmemWordsComp : kSceneSmemWords) * sizeof(float);
-}
-
 namespace {
 
 // Resident environments per SM of the per-world launch (0: as many as the
 // registers allow).  NUMI_B200_SCENE_RESIDENT, read once, overrides it; a
-// lower count is reached by asking each one-warp CTA for more shared memory.
+// lower count is reached by asking each CTA for more shared memory.
 int scene_resident_limit() {
     static const int limit = [] {
         const char* env = std::getenv("NUMI_B200_SCENE_RESIDENT");
@@ -99,17 +79,47 @@ int scene_resident_limit() {
     return limit;
 }
 
-size_t scene_launch_smem(bool compensated) {
-    size_t smem = scene_step_smem_bytes(compensated);
+// Warps and shared memory (floats) of a launch over `envs` environments of
+// `nb` bodies.  The registers hold 16 warps per SM.  Four warps per
+// environment finish one soonest, so that is the shape while every
+// environment is resident at once (4 per SM); past that, fewer warps waste
+// less on barriers and idle lanes, and small worlds do best with one.
+// Measured, us per control step (start of the table: 1 / 2 / 4 warps):
+//   pile    9 bodies:  500 envs 229 / 216 / 205;  8000 envs 1246 / 1983 / 2565
+//   pile   20 bodies:  500 envs 318 / 239 / 213;  8000 envs 1852 / 2347 / 2947
+//   pile   36 bodies:  16384 envs 7292 / 6598 / 6813
+//   pile   47 bodies:  500 envs 652 / 374 / 278;  8000 envs 4368 / 3255 / 3612
+//   pile   61 bodies:  500 envs 837 / 527 / 362;  8000 envs 5243 / 4562 / 4695
+// Support-mapped worlds keep per-thread polytopes in local memory, which
+// wants the L1 more than residency: 49-body hull piles, 1500 envs, 864 / 944
+// / 694; 23-body cylinder piles, 3000 envs, 1009 / 1030 / 1222.
+// Shared memory: no more than a shape uses, because what it leaves is L1.
+SceneShape scene_shape(int nb, int envs, bool compensated, bool convex) {
+    SceneShape shape{};
+    constexpr int kSmall = 28;   // bodies
+    constexpr int kResidentFour = 4 * 148, kResidentTwo = 8 * 148;
+    int total = 7000;
+    if (envs <= kResidentFour || (convex && nb > kSmall)) {
+        shape.warps = 4;
+    } else if (nb > kSmall) {
+        shape.warps = 2;
+    } else {
+        shape.warps = envs <= kResidentTwo ? 2 : 1;
+        total = convex && shape.warps == 1 ? 2800 : 3370;
+    }
+    const int words = std::max(kUnionLeast, std::min(kUnionMost, total - scene_smem_words(nb, 0, compensated)));
+    shape.smem = static_cast<size_t>(scene_smem_words(nb, words, compensated)) * sizeof(float);
     if (const int limit = scene_resident_limit()) {
-        int dev = 0, per_sm = 0;
+        int dev = 0, per_sm = 0, per_block = 0;
         if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess && per_sm > 0) {
-            const size_t padded = static_cast<size_t>(per_sm / limit) - 1024;  // 1 KB reserved per CTA
-            if (padded > smem) smem = padded;
+            cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess && per_sm > 0 &&
+            cudaDeviceGetAttribute(&per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess) {
+            // 1 KB reserved per CTA
+            const size_t padded = std::min(static_cast<size_t>(per_sm / limit) - 1024, static_cast<size_t>(per_block));
+            if (padded > shape.smem) shape.smem = padded;
         }
     }
-    return smem;
+    return shape;
 }
 
 }  // namespace
@@ -126,15 +136,17 @@ cudaError_t for_scene_kernel(bool compensated, bool convex, F&& f) {
 }  // namespace
 
 cudaError_t configure_scene_step_kernel() {
-    // The driver's default carveout keeps most of the unified L1 as cache,
-    // which the narrowphase scratch and contact records rely on.
+    // The driver's default carveout keeps the rest of the unified L1 as
+    // cache, which the manifold tables rely on.
     cudaError_t e = cudaSuccess;
     for (const bool compensated : {false, true})
         for (const bool convex : {false, true})
             if (e == cudaSuccess)
                 e = for_scene_kernel(compensated, convex, [&](auto kernel) {
-                    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                static_cast<int>(scene_launch_smem(compensated)));
+                    int dev = 0, per_block = 0;
+                    cudaError_t q = cudaGetDevice(&dev);
+                    if (q == cudaSuccess) q = cudaDeviceGetAttribute(&per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+                    return q != cudaSuccess ? q : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, per_block);
                 });
     return e;
 }
@@ -145,23 +157,27 @@ cudaError_t configure_mix_scene_kernel(bool convex, size_t max_dynamic_smem) {
                   : cudaFuncSetAttribute(mix_scene_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-cudaError_t mix_scene_occupancy(bool convex, int warps_per_block, size_t smem_per_block, int* blocks_per_sm) {
-    return convex ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, mix_scene_kernel<true>, 32 * warps_per_block,
-                                                                  smem_per_block)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, mix_scene_kernel<false>, 32 * warps_per_block,
-                                                                  smem_per_block);
+// A batch ends with its longest environments, so it takes the shape that
+// finishes one soonest; room for a full block of pairs at any body count.
+// 4000-environment mix: 7633 us with one warp, 5715 with two, 5143 with four
+// (5329 in 7000 floats).
+int mix_scene_warps() { return kSceneMaxWarps; }
+size_t mix_scene_smem_bytes() { return size_t(10200) * sizeof(float); }
+
+cudaError_t mix_scene_occupancy(bool convex, size_t smem_per_block, int* blocks_per_sm) {
+    const int threads = 32 * mix_scene_warps();
+    return convex ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, mix_scene_kernel<true>, threads, smem_per_block)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, mix_scene_kernel<false>, threads, smem_per_block);
 }
 
 cudaError_t launch_mix_scene(bool convex, const MixWorld* worlds, int world_count, int steps, const std::uint32_t* items,
-                             int item_count, unsigned* next_item, int warps_per_block, int smem_floats_per_warp, int grid,
-                             cudaStream_t stream) {
-    const size_t smem = static_cast<size_t>(smem_floats_per_warp) * sizeof(float) * warps_per_block;
+                             int item_count, unsigned* next_item, size_t smem_per_block, int grid, cudaStream_t stream) {
+    if (smem_per_block < mix_scene_smem_bytes()) return cudaErrorInvalidValue;
+    const int threads = 32 * mix_scene_warps();
     if (convex)
-        mix_scene_kernel<true><<<grid, 32 * warps_per_block, smem, stream>>>(worlds, world_count, steps, items, item_count, next_item,
-                                                                             smem_floats_per_warp);
+        mix_scene_kernel<true><<<grid, threads, smem_per_block, stream>>>(worlds, world_count, steps, items, item_count, next_item);
     else
-        mix_scene_kernel<false><<<grid, 32 * warps_per_block, smem, stream>>>(worlds, world_count, steps, items, item_count, next_item,
-                                                                              smem_floats_per_warp);
+        mix_scene_kernel<false><<<grid, threads, smem_per_block, stream>>>(worlds, world_count, steps, items, item_count, next_item);
     return cudaGetLastError();
 }
 
@@ -172,9 +188,10 @@ cudaError_t launch_scene_audit(const SceneParams& p, cudaStream_t stream) {
 
 cudaError_t launch_scene_step(const SceneParams& p, cudaStream_t stream) {
     const bool compensated = p.q_comp != nullptr;
-    const size_t smem = scene_launch_smem(compensated);
+    if (p.bodies < 1 || p.bodies > kSceneMaxBodies) return cudaErrorInvalidValue;
+    const SceneShape shape = scene_shape(p.bodies, p.env_count, compensated, p.support_mapped != 0);
     return for_scene_kernel(compensated, p.support_mapped != 0, [&](auto kernel) {
-        kernel<<<p.env_count, 32, smem, stream>>>(p);
+        kernel<<<p.env_count, 32 * shape.warps, shape.smem, stream>>>(p);
         return cudaGetLastError();
     });
 }

@@ -1,9 +1,10 @@
 // Free-body control step on B200 -- device code shared by the per-world
-// kernel (scene_step.cu) and the heterogeneous batch kernel (mix_step.cu):
-// piles of spheres, capsules, boxes and cylinders on a ground plane
-// (numi-lab's scene bodies).  One warp per environment for a whole
-// control step; lanes own bodies (two per lane), compiled pairs, candidate
-// pairs, manifolds and contacts in turn.
+// kernel and the heterogeneous batch kernel (scene_step.cu): piles of
+// spheres, capsules, boxes, cylinders and convex hulls on a ground plane
+// (numi-lab's scene bodies).  One CTA per environment for a whole control
+// step; its threads own bodies, compiled pairs, candidate pairs, manifolds
+// and contacts in turn, and everything a sweep reads lives in shared memory
+// or registers.
 //
 // Stage order per substep follows the reference's MetalWorld graph for scene
 // bodies: prediction (mr_world_predict_scene, MetalWorldContact.metal:
@@ -43,85 +44,105 @@ constexpr int kRawCap = 8;
 // (the first axis wins).  The FP64 CPU collision uses 1e-24 and 1e-12.
 constexpr float kParallelEdges = 1.0e-12f;
 constexpr float kAxisTie = 1.0e-7f;
-constexpr int kRecWords = 16;                                   // candidate record
-constexpr int kLaneScratch = (4 + kRawCap) * kRecWords + 4;  // records, candidate ids
-constexpr int kCw = 40;                                          // contact record words
+// Narrowphase scratch of one candidate pair in shared memory: its class's
+// raw contact records (anchors in the bodies' frames, features, world
+// midpoint, separation), the midpoint and separation of the four old points,
+// and the pair's normal.
+constexpr int kRawWords = 12;
+constexpr int kOldWords = 4;
+constexpr int kPairFixed = 4 * kOldWords + 3;
+// Candidate pairs whose narrowphase and manifolds are built together, one
+// per lane (at most 32 on one warp), spread evenly over the CTA's warps, as
+// many as the scratch holds.  Within a block they are sorted into cost groups: the narrowphase
+// classes diverge, so a warp of mixed pairs pays for every class in it, one
+// after the other.
+constexpr int kPairBlock = 64;
+constexpr int kPairGroups = 4;
+// Contact rows a thread keeps in registers, and the words of one row in the
+// workspace, where a thread's further rows live.
+constexpr int kOwnRows = 2;
+constexpr int kRowWords = 25;
 
-// Shared-memory layout of one environment (floats): body state, swept
-// bounds, candidate pairs and per-body contact lists -- about 9 KB, so that
-// registers, not shared memory, bound the resident warps.
-constexpr int kOffPos = 0;
-constexpr int kOffQuat = kOffPos + kSceneMaxBodies * 3;
-constexpr int kOffLin = kOffQuat + kSceneMaxBodies * 4;
-constexpr int kOffAng = kOffLin + kSceneMaxBodies * 3;
-constexpr int kOffIiw = kOffAng + kSceneMaxBodies * 3;   // world inverse inertia, sym 6
-constexpr int kOffLo = kOffIiw + kSceneMaxBodies * 6;
-constexpr int kOffHi = kOffLo + kSceneMaxBodies * 3;
-constexpr int kOffMargin = kOffHi + kSceneMaxBodies * 3;
-// Candidate pairs (u16) live only until the narrowphase has consumed them;
-// the per-body contact list entries (u16) reuse their words afterwards.
-constexpr int kOffCand = kOffMargin + kSceneMaxBodies;
-constexpr int kOffEntries = kOffCand;
+// Shared-memory layout of one environment of nb bodies (floats): body state,
+// swept bounds, candidate pairs and per-body contact lists, then a union: the
+// pair flags of the broadphase, the narrowphase scratch, and the contact
+// arrays once the manifolds are built.  The union takes what the launch's
+// shared memory leaves; contact arrays that do not fit it live in the
+// workspace for that substep.
+__host__ __device__ constexpr int off_pos(int) { return 0; }
+__host__ __device__ constexpr int off_quat(int nb) { return 3 * nb; }
+__host__ __device__ constexpr int off_lin(int nb) { return 7 * nb; }
+__host__ __device__ constexpr int off_ang(int nb) { return 10 * nb; }
+__host__ __device__ constexpr int off_iiw(int nb) { return 13 * nb; }  // world inverse inertia, sym 6
+__host__ __device__ constexpr int off_lo(int nb) { return 19 * nb; }   // swept bounds; later the manifolds of each body (128-bit sets)
+__host__ __device__ constexpr int off_hi(int nb) { return 22 * nb; }
+__host__ __device__ constexpr int off_margin(int nb) { return 25 * nb; }
+__host__ __device__ constexpr int off_im(int nb) { return 26 * nb; }   // inverse masses
+__host__ __device__ constexpr int off_fixed(int nb) { return 27 * nb; }
+// Offsets past off_fixed.  Candidate pairs (u16) live only until the
+// narrowphase has consumed them; the per-body contact list entries (u16)
+// reuse their words afterwards.
+constexpr int kOffCand = 0;
 constexpr int kCandWords = (kSceneCandidates > 2 * kSceneContacts ? kSceneCandidates : 2 * kSceneContacts) / 2;
-constexpr int kOffLists = kOffCand + kCandWords;  // start[65], fill[65] (ints)
-constexpr int kOffKeys = kOffLists + 2 * (kSceneMaxBodies + 1);  // pair keys of the two tables (u32)
-constexpr int kOffFirst = kOffKeys + 2 * kSceneManifolds;  // first contact of each manifold (u16, +1)
-constexpr int kOffMisc = kOffFirst + (kSceneManifolds + 2) / 2;
-constexpr int kSceneSmemWords = kOffMisc + 32;
-// Compensated precision only, past the FP32 layout: compensation terms of
-// the body positions' running sums (persistent, [env][body][7] entries 0-2
-// in HBM) and of the substep's velocity sums over the Jacobi sweeps.
-constexpr int kOffPosComp = kSceneSmemWords;
-constexpr int kOffLinComp = kOffPosComp + kSceneMaxBodies * 3;
-constexpr int kOffAngComp = kOffLinComp + kSceneMaxBodies * 3;
-constexpr int kSceneSmemWordsComp = kOffAngComp + kSceneMaxBodies * 3;
+constexpr int kOffLists = kOffCand + kCandWords;  // start of each body's contact list (ints, +1)
+constexpr int kOffKeys = kOffLists + kSceneMaxBodies + 1;  // pair keys of the two tables (u16)
+constexpr int kOffFirst = kOffKeys + kSceneManifolds;      // first contact of each manifold (u16, +1)
+constexpr int kOffAb = kOffFirst + (kSceneManifolds + 2) / 2;  // bodies of each manifold (u16: a << 8 | b)
+constexpr int kOffMap = kOffAb + kSceneManifolds / 2;       // manifold * 4 + point of each contact (u16)
+constexpr int kOffCab = kOffMap + kSceneContacts / 2;       // bodies of each contact (u16: a << 8 | b)
+constexpr int kOffSorted = kOffCab + kSceneContacts / 2;    // a block's pairs in group order (bytes)
+constexpr int kOffScratch = kOffSorted + kPairBlock / 4;    // and where their scratch starts (u16)
+constexpr int kOffMisc = kOffScratch + kPairBlock / 2;
+constexpr int kFixedWords = kOffMisc + 32;
+__host__ __device__ constexpr int off_union(int nb) { return off_fixed(nb) + kFixedWords; }
+// Contact arrays [contact][3]: normals until the rows exist, then impulse
+// changes of the sweep; and the contact point relative to both bodies.
+constexpr int kContactArrays = 9;
+// Compensated precision only, at the end: compensation terms of the body
+// positions' running sums (persistent, [env][body][7] entries 0-2 in HBM)
+// and of the substep's velocity sums over the Jacobi sweeps.
+__host__ __device__ constexpr int comp_words(int nb, bool compensated) { return compensated ? 9 * nb : 0; }
+// Words of shared memory with a union of `words`.
+__host__ __device__ constexpr int scene_smem_words(int nb, int words, bool compensated) {
+    return off_union(nb) + words + comp_words(nb, compensated);
+}
+constexpr int kUnionLeast = (kSceneMaxPairs + 31) / 32 > kRawCap * kRawWords + kPairFixed ? (kSceneMaxPairs + 31) / 32 : kRawCap * kRawWords + kPairFixed;
+constexpr int kUnionMost = kPairBlock * (kRawCap * kRawWords + kPairFixed) > kContactArrays * kSceneContacts
+                               ? kPairBlock * (kRawCap * kRawWords + kPairFixed) : kContactArrays * kSceneContacts;
+__device__ __forceinline__ int dynamic_smem_words() {
+    unsigned bytes;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(bytes));
+    return static_cast<int>(bytes / sizeof(float));
+}
 
-// Global workspace of one environment (floats, L2-resident while the
-// environment runs): two substep manifold tables, the contact records and
-// one narrowphase scratch block per lane.
+// Global workspace of one environment (floats): two substep manifold tables,
+// the rows of contacts past kOwnRows per thread, and the contact arrays of a
+// substep whose contacts do not fit shared memory.
 constexpr int kTableWords = kSceneManifolds * kSceneSlotWords;
 constexpr int kWsTable0 = 0;
 constexpr int kWsTable1 = kWsTable0 + kTableWords;
-constexpr int kWsContacts = kWsTable1 + kTableWords;
-constexpr int kWsLanes = kWsContacts + kSceneContacts * kCw;
-constexpr int kWsWords = (kWsLanes + 32 * kLaneScratch + 31) / 32 * 32;
+constexpr int kWsRows = kWsTable1 + kTableWords;
+constexpr int kWsArrays = kWsRows + kSceneContacts * kRowWords;
+constexpr int kWsWords = (kWsArrays + kSceneContacts * kContactArrays + 31) / 32 * 32;
 
-enum SceneMisc : int { kSmStatus = 0, kSmFail = 1, kSmContacts = 2, kSmManifolds = 3, kSmRaw = 4, kSmCand = 5, kSmIslands = 6 };
-enum SceneCw : int {
-    kScA = 0, kScB = 1, kScRa = 2, kScRb = 5, kScN = 8, kScT = 11, kScBt = 14, kScTarget = 17, kScReg = 20, kScMu = 21,
-    kScLambda = 22, kScPre = 25, kScRelax = 34, kScDelta = 35, kScSlot = 38, kScFlags = 39
+// Shared counters: the lowest failure of the phase (kSmStatus), the last
+// substep's contacts, the largest manifold, raw contact, candidate and
+// island counts, this substep's raw contacts, and the pairs with contacts of
+// this block and the next (bit sets).
+enum SceneMisc : int {
+    kSmStatus = 0, kSmContacts = 1, kSmManifolds = 2, kSmRaw = 3, kSmCand = 4, kSmIslands = 5, kSmRawNow = 6, kSmTouching = 8
 };
-enum CandWord : int { kCdLaS = 0, kCdLbS = 3, kCdFaS = 6, kCdFbS = 7, kCdWpS = 8, kCdSepS = 11, kCdLifeS = 12, kCdImpS = 13 };
+// Raw records: local anchors on A and B, features, world midpoint, separation.
+enum RawWord : int { kRwLa = 0, kRwLb = 3, kRwFa = 6, kRwFb = 7, kRwWp = 8, kRwSep = 11 };
 
 __device__ __forceinline__ int ai(float f) { return __float_as_int(f); }
 __device__ __forceinline__ float af(int i) { return __int_as_float(i); }
 
-// One contact record.  Records are stored word-major ([word][contact]), so
-// the lanes of a warp reading one word of consecutive contacts touch one
-// cache line.
-struct Rec {
-    float* p;
-    __device__ __forceinline__ float& operator[](int w) const { return p[w * kSceneContacts]; }
-    __device__ __forceinline__ float3 v3(int w) const {
-        return f3(p[w * kSceneContacts], p[(w + 1) * kSceneContacts], p[(w + 2) * kSceneContacts]);
-    }
-    __device__ __forceinline__ void set3(int w, float3 v) const {
-        p[w * kSceneContacts] = v.x;
-        p[(w + 1) * kSceneContacts] = v.y;
-        p[(w + 2) * kSceneContacts] = v.z;
-    }
-};
-__device__ __forceinline__ Rec rec(float* C, int c) { return Rec{C + c}; }
-
-__device__ __forceinline__ void fail(float* misc, unsigned code, unsigned index) {
-    if (ai(misc[kSmStatus]) == MR_STEP_SUCCESS) {
-        misc[kSmStatus] = af(static_cast<int>(code));
-        misc[kSmFail] = af(static_cast<int>(index));
-    }
-}
-__device__ __forceinline__ bool ok(const float* misc) {
-    __syncwarp();
-    return ai(misc[kSmStatus]) == MR_STEP_SUCCESS;
+// Records a failure of the current phase; the lowest rank wins, so the code
+// does not depend on the order of the threads.
+constexpr unsigned kNoFailure = 0xffffffffu;
+__device__ __forceinline__ void fail(float* misc, unsigned rank, unsigned code) {
+    atomicMin(reinterpret_cast<unsigned*>(misc) + kSmStatus, (rank << 16) | code);
 }
 
 // World collider of a body or of the ground plane (index nb).
@@ -144,7 +165,8 @@ struct Collider {
 };
 
 __device__ void load_collider(const SceneModel& M, const float* s, int b, Collider& o) {
-    if (b >= M.nb) {
+    const int nb = M.nb;
+    if (b >= nb) {
         o.type = MR_SHAPE_PLANE;
         o.c = xyz(M.plane_position);
         o.r = M.plane_rotation;
@@ -163,14 +185,14 @@ __device__ void load_collider(const SceneModel& M, const float* s, int b, Collid
         return;
     }
     o.type = M.shape_type[b];
-    o.c = ld3(s + kOffPos + b * 3);
-    o.r = ld4(s + kOffQuat + b * 4);
+    o.c = ld3(s + off_pos(nb) + b * 3);
+    o.r = ld4(s + off_quat(nb) + b * 4);
     const float4 d = M.dims[b];
     o.half = xyz(d);
     o.radius = d.x;
-    o.offset = M.offsets[b].x + s[kOffMargin + b];
-    o.lo = ld3(s + kOffLo + b * 3);
-    o.hi = ld3(s + kOffHi + b * 3);
+    o.offset = M.offsets[b].x + s[off_margin(nb) + b];
+    o.lo = ld3(s + off_lo(nb) + b * 3);
+    o.hi = ld3(s + off_hi(nb) + b * 3);
     if (o.type == MR_SHAPE_CAPSULE) {
         const float3 axis = qrot(o.r, f3(0.0f, d.y, 0.0f));
         o.e0 = o.c - axis;
@@ -209,9 +231,13 @@ __device__ __forceinline__ float collider_scale(const Collider& k) {
 __device__ __forceinline__ float3 box_axis(const Collider& b, int axis) {
     return qrot(b.r, f3(axis == 0 ? 1.0f : 0.0f, axis == 1 ? 1.0f : 0.0f, axis == 2 ? 1.0f : 0.0f));
 }
-__device__ __forceinline__ float box_radius(const Collider& b, float3 axis) {
-    return fabsf(dot3(axis, box_axis(b, 0))) * b.half.x + fabsf(dot3(axis, box_axis(b, 1))) * b.half.y +
-           fabsf(dot3(axis, box_axis(b, 2))) * b.half.z;
+// A box's three axes, rotated once per pair.
+struct BoxAxes {
+    float3 x, y, z;
+    __device__ __forceinline__ float3 operator[](int a) const { return a == 0 ? x : (a == 1 ? y : z); }
+};
+__device__ __forceinline__ float box_radius(const Collider& b, const BoxAxes& ax, float3 axis) {
+    return fabsf(dot3(axis, ax.x)) * b.half.x + fabsf(dot3(axis, ax.y)) * b.half.y + fabsf(dot3(axis, ax.z)) * b.half.z;
 }
 __device__ __forceinline__ float3 box_vertex(const Collider& b, int v) {
     return b.c + qrot(b.r, f3((v & 1) ? b.half.x : -b.half.x, (v & 2) ? b.half.y : -b.half.y, (v & 4) ? b.half.z : -b.half.z));
@@ -367,6 +393,7 @@ __device__ __forceinline__ CapsuleBoxWitness capsule_box_witness(float3 ce0, flo
             best_f = f;
         }
     };
+#pragma unroll 1
     for (int e = 0; e < 2; ++e) {
         const float3 sp = e == 0 ? s0 : s1;
         consider(sp, f3(fminf(fmaxf(sp.x, -he[0]), he[0]), fminf(fmaxf(sp.y, -he[1]), he[1]), fminf(fmaxf(sp.z, -he[2]), he[2])),
@@ -375,6 +402,7 @@ __device__ __forceinline__ CapsuleBoxWitness capsule_box_witness(float3 ce0, flo
     unsigned feature = 2u;
     for (int va = 0; va < 3; ++va) {
         const int f0 = (va + 1) % 3, f1 = (va + 2) % 3;
+#pragma unroll 1
         for (int sg = 0; sg < 4; ++sg) {
             float c0[3], c1[3];
             c0[va] = -he[va];
@@ -409,13 +437,13 @@ struct RawSink {
     float4 rotA, rotB;
     __device__ void add(float3 pa, float3 pb, float sep, unsigned fa, unsigned fb) {
         if (count >= kRawCap) return;
-        float* r = rec + count * kRecWords;
-        st3(r + kCdLaS, qrotinv(rotA, pa - posA));
-        st3(r + kCdLbS, qrotinv(rotB, pb - posB));
-        r[kCdFaS] = af(static_cast<int>(fa));
-        r[kCdFbS] = af(static_cast<int>(fb));
-        st3(r + kCdWpS, 0.5f * (pa + pb));
-        r[kCdSepS] = sep;
+        float* r = rec + count * kRawWords;
+        st3(r + kRwLa, qrotinv(rotA, pa - posA));
+        st3(r + kRwLb, qrotinv(rotB, pb - posB));
+        r[kRwFa] = af(static_cast<int>(fa));
+        r[kRwFb] = af(static_cast<int>(fb));
+        st3(r + kRwWp, 0.5f * (pa + pb));
+        r[kRwSep] = sep;
         ++count;
     }
 };
@@ -487,6 +515,7 @@ __device__ float3 shape_support(const Collider& k, unsigned index, float3 d, uns
         const float3 l = qrotinv(k.r, d);
         float best = -INFINITY;
         int bi = 0;
+#pragma unroll 1
         for (int i = 0; i < k.hull_count; ++i) {
             const float4 v = k.hull[i];
             const float pr = dot3(f3(v.x, v.y, v.z), l);
@@ -594,14 +623,18 @@ __device__ void compress_simplex(Sup* sx, int& n, float* wt) {
     Sup keep[4];
     float kw[4];
     int m = 0, best = 0;
+#pragma unroll 1
     for (int i = 1; i < n; ++i)
         if (wt[i] > wt[best]) best = i;
+#pragma unroll 1
     for (int i = 0; i < n; ++i)
         if (wt[i] > 1.0e-7f) { keep[m] = sx[i]; kw[m] = wt[i]; ++m; }
     if (m == 0) { keep[0] = sx[best]; kw[0] = 1.0f; m = 1; }
     float tot = 0.0f;
+#pragma unroll 1
     for (int i = 0; i < m; ++i) tot += kw[i];
     const float inv = tot > kTinyS ? 1.0f / tot : 1.0f;
+#pragma unroll 1
     for (int i = 0; i < m; ++i) { sx[i] = keep[i]; wt[i] = kw[i] * inv; }
     n = m;
 }
@@ -639,6 +672,7 @@ __device__ bool closest_simplex(Sup* sx, int& n, float* wt, float3& closest) {
     const int faces[4][3] = {{0, 1, 2}, {0, 3, 1}, {0, 2, 3}, {1, 3, 2}};
     float best = INFINITY, bw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     float3 bp = f3(0.0f, 0.0f, 0.0f);
+#pragma unroll 1
     for (int f = 0; f < 4; ++f) {
         float tw[3];
         const float3 p = closest_triangle(sx[faces[f][0]].w, sx[faces[f][1]].w, sx[faces[f][2]].w, tw);
@@ -651,15 +685,20 @@ __device__ bool closest_simplex(Sup* sx, int& n, float* wt, float3& closest) {
         }
     }
     closest = bp;
+#pragma unroll 1
     for (int i = 0; i < 4; ++i) wt[i] = bw[i];
     compress_simplex(sx, n, wt);
     return false;
 }
 
 // GJK distance: returns 1 on overlap (the simplex seeds EPA), 0 apart (q
-// holds the witness), -1 without convergence.
-__device__ int gjk(const Collider& A, const Collider& B, unsigned ia, unsigned ib, float scale, Sup* sx, int& n, float* wt,
-                   SmQuery& q) {
+// holds the witness), 2 apart by more than `accepted` (q is not set), -1
+// without convergence.  Each support bounds the distance from below by its
+// projection on the search direction; most candidate pairs -- bounds that
+// touch, shapes that do not -- are rejected by that bound after one or two
+// supports, where the witness takes five to ten.
+__device__ int gjk(const Collider& A, const Collider& B, unsigned ia, unsigned ib, float scale, float accepted, Sup* sx, int& n,
+                   float* wt, SmQuery& q) {
     const float tol = 32.0f * kFltEps * scale;
     float3 d = B.c - A.c;
     if (dot3(d, d) <= kTinyS) d = deterministic_direction(ia * 65537u + ib);
@@ -673,6 +712,12 @@ __device__ int gjk(const Collider& A, const Collider& B, unsigned ia, unsigned i
         d = -closest;
         Sup cand;
         minkowski(A, B, ia, ib, d, cand);
+        // A margin of tol keeps the decision that of the converged distance,
+        // which is never below the bound.  (Explicit roundings: sharing these
+        // products with `advance` would change how that one is contracted.)
+        const float against = -__fmaf_rn(cand.w.x, d.x, __fmaf_rn(cand.w.y, d.y, __fmul_rn(cand.w.z, d.z)));
+        const float dd = __fmaf_rn(d.x, d.x, __fmaf_rn(d.y, d.y, __fmul_rn(d.z, d.z)));
+        if (against > 0.0f && __fmul_rn(against, against) > __fmul_rn(__fmul_rn(accepted + tol, accepted + tol), dd)) return 2;
         bool dup = false;
         for (int i = 0; i < n; ++i) {
             const float3 e = cand.w - sx[i].w;
@@ -981,7 +1026,8 @@ __device__ __noinline__ unsigned support_mapped_contacts(const Collider& A, cons
     int n = 0;
     SmQuery q;
     q.normal = f3(0.0f, 0.0f, 1.0f);
-    const int g = gjk(A, B, ia, ib, scale, sx, n, wt, q);
+    const int g = gjk(A, B, ia, ib, scale, accepted, sx, n, wt, q);
+    if (g == 2) return MR_STEP_SUCCESS;
     if (hull) {
         if (g != 0 && !support_axis_witness(A, B, ia, ib, q)) return MR_STEP_DID_NOT_CONVERGE;
     } else if (g == 1) {
@@ -1055,114 +1101,115 @@ __device__ __noinline__ unsigned support_mapped_contacts(const Collider& A, cons
 // Returns MR_STEP_SUCCESS, or the code of a support-mapped query that did
 // not resolve.
 template <bool kConvex>
-__device__ unsigned narrowphase(const Collider& A, const Collider& B, int cls, unsigned ia, unsigned ib, float accepted,
+__device__ __forceinline__ unsigned narrowphase(const Collider& A, const Collider& B, int cls, unsigned ia, unsigned ib, float accepted,
                                 RawSink& sink, float3& normal) {
     if constexpr (kConvex) {
         if (cls == MR_COLLISION_PAIR_CONVEX) return support_mapped_contacts(A, B, ia, ib, accepted, sink, normal);
     }
-    if (cls == MR_COLLISION_PAIR_SPHERE_SPHERE) {
-        const float3 delta = B.c - A.c;
-        const float d = len3(delta);
-        normal = d > kTinyS ? delta * (1.0f / d) : coincident_normal(ia, ib);
-        const float sep = d - A.radius - B.radius;
-        if (sep <= accepted)
-            sink.add(A.c + normal * A.radius, B.c - normal * B.radius, sep, feature_key(MR_SHAPE_SPHERE, 0u),
-                     feature_key(MR_SHAPE_SPHERE, 0u));
-        return MR_STEP_SUCCESS;
-    }
-    if (cls == MR_COLLISION_PAIR_SPHERE_BOX) {
-        const bool sphere_a = A.type == MR_SHAPE_SPHERE;
-        const Collider& sp = sphere_a ? A : B;
-        const Collider& bx = sphere_a ? B : A;
-        const float3 lc = qrotinv(bx.r, sp.c - bx.c);
-        float3 cl = f3(fminf(fmaxf(lc.x, -bx.half.x), bx.half.x), fminf(fmaxf(lc.y, -bx.half.y), bx.half.y),
-                       fminf(fmaxf(lc.z, -bx.half.z), bx.half.z));
-        const float3 ld = cl - lc;
-        const float dist = len3(ld);
-        float3 n;
+    // One contact from the closest points of two round shapes or a round
+    // shape and a box: each class finds them, one append follows.
+    if (cls != MR_COLLISION_PAIR_BOX_BOX && B.type != MR_SHAPE_PLANE) {
+        float3 pa, pb;
         float sep;
-        unsigned feat;
-        if (dist > kTinyS) {
-            n = qrot(bx.r, ld * (1.0f / dist));
-            sep = dist - sp.radius;
-            auto region = [](float c, float he) { return c < -he ? 0u : (c > he ? 2u : 1u); };
-            feat = region(lc.x, bx.half.x) + 3u * region(lc.y, bx.half.y) + 9u * region(lc.z, bx.half.z);
-        } else {
-            const float dx = bx.half.x - fabsf(lc.x), dy = bx.half.y - fabsf(lc.y), dz = bx.half.z - fabsf(lc.z);
-            int axis = 0;
-            float dm = dx;
-            if (dy < dm) { axis = 1; dm = dy; }
-            if (dz < dm) { axis = 2; dm = dz; }
-            const float coord = axis == 0 ? lc.x : (axis == 1 ? lc.y : lc.z);
-            const float sign = coord >= 0.0f ? 1.0f : -1.0f;
-            const float3 outward = f3(axis == 0 ? sign : 0.0f, axis == 1 ? sign : 0.0f, axis == 2 ? sign : 0.0f);
-            if (axis == 0) cl.x = sign * bx.half.x;
-            else if (axis == 1) cl.y = sign * bx.half.y;
-            else cl.z = sign * bx.half.z;
-            n = qrot(bx.r, -outward);
-            sep = -dm - sp.radius;
-            feat = 27u + 2u * static_cast<unsigned>(axis) + (sign > 0.0f ? 1u : 0u);
-        }
-        const float3 box_point = bx.c + qrot(bx.r, cl);
-        if (sep <= accepted) {
+        unsigned fa, fb;
+        if (cls == MR_COLLISION_PAIR_SPHERE_SPHERE) {
+            const float3 delta = B.c - A.c;
+            const float d = len3(delta);
+            normal = d > kTinyS ? delta * (1.0f / d) : coincident_normal(ia, ib);
+            sep = d - A.radius - B.radius;
+            pa = A.c + normal * A.radius;
+            pb = B.c - normal * B.radius;
+            fa = fb = feature_key(MR_SHAPE_SPHERE, 0u);
+        } else if (cls == MR_COLLISION_PAIR_SPHERE_BOX) {
+            const bool sphere_a = A.type == MR_SHAPE_SPHERE;
+            const Collider& sp = sphere_a ? A : B;
+            const Collider& bx = sphere_a ? B : A;
+            const float3 lc = qrotinv(bx.r, sp.c - bx.c);
+            float3 cl = f3(fminf(fmaxf(lc.x, -bx.half.x), bx.half.x), fminf(fmaxf(lc.y, -bx.half.y), bx.half.y),
+                           fminf(fmaxf(lc.z, -bx.half.z), bx.half.z));
+            const float3 ld = cl - lc;
+            const float dist = len3(ld);
+            float3 n;
+            unsigned feat;
+            if (dist > kTinyS) {
+                n = qrot(bx.r, ld * (1.0f / dist));
+                sep = dist - sp.radius;
+                auto region = [](float c, float he) { return c < -he ? 0u : (c > he ? 2u : 1u); };
+                feat = region(lc.x, bx.half.x) + 3u * region(lc.y, bx.half.y) + 9u * region(lc.z, bx.half.z);
+            } else {
+                const float dx = bx.half.x - fabsf(lc.x), dy = bx.half.y - fabsf(lc.y), dz = bx.half.z - fabsf(lc.z);
+                int axis = 0;
+                float dm = dx;
+                if (dy < dm) { axis = 1; dm = dy; }
+                if (dz < dm) { axis = 2; dm = dz; }
+                const float coord = axis == 0 ? lc.x : (axis == 1 ? lc.y : lc.z);
+                const float sign = coord >= 0.0f ? 1.0f : -1.0f;
+                const float3 outward = f3(axis == 0 ? sign : 0.0f, axis == 1 ? sign : 0.0f, axis == 2 ? sign : 0.0f);
+                if (axis == 0) cl.x = sign * bx.half.x;
+                else if (axis == 1) cl.y = sign * bx.half.y;
+                else cl.z = sign * bx.half.z;
+                n = qrot(bx.r, -outward);
+                sep = -dm - sp.radius;
+                feat = 27u + 2u * static_cast<unsigned>(axis) + (sign > 0.0f ? 1u : 0u);
+            }
+            const float3 box_point = bx.c + qrot(bx.r, cl);
             const float3 sphere_point = sp.c + n * sp.radius;
-            if (sphere_a)
-                sink.add(sphere_point, box_point, sep, feature_key(MR_SHAPE_SPHERE, 0u), feature_key(MR_SHAPE_BOX, feat));
-            else
-                sink.add(box_point, sphere_point, sep, feature_key(MR_SHAPE_BOX, feat), feature_key(MR_SHAPE_SPHERE, 0u));
-        }
-        normal = sphere_a ? n : -n;
-        return MR_STEP_SUCCESS;
-    }
-    if (cls == MR_COLLISION_PAIR_SPHERE_CAPSULE) {
-        const bool sphere_a = A.type == MR_SHAPE_SPHERE;
-        const Collider& sp = sphere_a ? A : B;
-        const Collider& cp = sphere_a ? B : A;
-        float t;
-        const float3 on = closest_on_segment(sp.c, cp.e0, cp.e1, t);
-        const float3 delta = on - sp.c;
-        const float d = len3(delta);
-        const float3 n = d > kTinyS ? delta * (1.0f / d)
-                                    : stable_segment_normal(cp.e1 - cp.e0, f3(0.0f, 0.0f, 0.0f), sphere_a ? ia : ib, sphere_a ? ib : ia);
-        const float sep = d - sp.radius - cp.radius;
-        if (sep <= accepted) {
+            const unsigned fs = feature_key(MR_SHAPE_SPHERE, 0u), fx = feature_key(MR_SHAPE_BOX, feat);
+            pa = sphere_a ? sphere_point : box_point;
+            pb = sphere_a ? box_point : sphere_point;
+            fa = sphere_a ? fs : fx;
+            fb = sphere_a ? fx : fs;
+            normal = sphere_a ? n : -n;
+        } else if (cls == MR_COLLISION_PAIR_SPHERE_CAPSULE) {
+            const bool sphere_a = A.type == MR_SHAPE_SPHERE;
+            const Collider& sp = sphere_a ? A : B;
+            const Collider& cp = sphere_a ? B : A;
+            float t;
+            const float3 on = closest_on_segment(sp.c, cp.e0, cp.e1, t);
+            const float3 delta = on - sp.c;
+            const float d = len3(delta);
+            const float3 n = d > kTinyS ? delta * (1.0f / d)
+                                        : stable_segment_normal(cp.e1 - cp.e0, f3(0.0f, 0.0f, 0.0f), sphere_a ? ia : ib, sphere_a ? ib : ia);
+            sep = d - sp.radius - cp.radius;
             const float3 ps = sp.c + n * sp.radius, pc = on - n * cp.radius;
             const unsigned fs = feature_key(MR_SHAPE_SPHERE, 0u), fc = feature_key(MR_SHAPE_CAPSULE, capsule_feature(t));
-            if (sphere_a) sink.add(ps, pc, sep, fs, fc);
-            else sink.add(pc, ps, sep, fc, fs);
+            pa = sphere_a ? ps : pc;
+            pb = sphere_a ? pc : ps;
+            fa = sphere_a ? fs : fc;
+            fb = sphere_a ? fc : fs;
+            normal = sphere_a ? n : -n;
+        } else if (cls == MR_COLLISION_PAIR_CAPSULE_CAPSULE) {
+            float3 ca, cb;
+            float ta, tb;
+            closest_segments(A.e0, A.e1, B.e0, B.e1, ca, cb, ta, tb);
+            const float3 delta = cb - ca;
+            const float d = len3(delta);
+            normal = d > kTinyS ? delta * (1.0f / d) : stable_segment_normal(A.e1 - A.e0, B.e1 - B.e0, ia, ib);
+            sep = d - A.radius - B.radius;
+            pa = ca + normal * A.radius;
+            pb = cb - normal * B.radius;
+            fa = feature_key(MR_SHAPE_CAPSULE, capsule_feature(ta));
+            fb = feature_key(MR_SHAPE_CAPSULE, capsule_feature(tb));
+        } else {  // capsule-box
+            const bool capsule_a = A.type == MR_SHAPE_CAPSULE;
+            const Collider& cp = capsule_a ? A : B;
+            const Collider& bx = capsule_a ? B : A;
+            const CapsuleBoxWitness w =
+                capsule_box_witness(cp.e0, cp.e1, cp.radius, bx.c, bx.r, bx.half, capsule_a ? ia : ib, capsule_a ? ib : ia);
+            const unsigned fc = feature_key(MR_SHAPE_CAPSULE, capsule_feature(w.t_cap)), fx = feature_key(MR_SHAPE_BOX, w.box_feature);
+            sep = w.sep;
+            pa = capsule_a ? w.cap_point : w.box_point;
+            pb = capsule_a ? w.box_point : w.cap_point;
+            fa = capsule_a ? fc : fx;
+            fb = capsule_a ? fx : fc;
+            normal = capsule_a ? w.normal : -w.normal;
         }
-        normal = sphere_a ? n : -n;
-        return MR_STEP_SUCCESS;
-    }
-    if (cls == MR_COLLISION_PAIR_CAPSULE_CAPSULE) {
-        float3 pa, pb;
-        float ta, tb;
-        closest_segments(A.e0, A.e1, B.e0, B.e1, pa, pb, ta, tb);
-        const float3 delta = pb - pa;
-        const float d = len3(delta);
-        normal = d > kTinyS ? delta * (1.0f / d) : stable_segment_normal(A.e1 - A.e0, B.e1 - B.e0, ia, ib);
-        const float sep = d - A.radius - B.radius;
-        if (sep <= accepted)
-            sink.add(pa + normal * A.radius, pb - normal * B.radius, sep, feature_key(MR_SHAPE_CAPSULE, capsule_feature(ta)),
-                     feature_key(MR_SHAPE_CAPSULE, capsule_feature(tb)));
-        return MR_STEP_SUCCESS;
-    }
-    if (cls == MR_COLLISION_PAIR_CAPSULE_BOX) {
-        const bool capsule_a = A.type == MR_SHAPE_CAPSULE;
-        const Collider& cp = capsule_a ? A : B;
-        const Collider& bx = capsule_a ? B : A;
-        const CapsuleBoxWitness w =
-            capsule_box_witness(cp.e0, cp.e1, cp.radius, bx.c, bx.r, bx.half, capsule_a ? ia : ib, capsule_a ? ib : ia);
-        if (w.sep <= accepted) {
-            const unsigned fc = feature_key(MR_SHAPE_CAPSULE, capsule_feature(w.t_cap)), fb = feature_key(MR_SHAPE_BOX, w.box_feature);
-            if (capsule_a) sink.add(w.cap_point, w.box_point, w.sep, fc, fb);
-            else sink.add(w.box_point, w.cap_point, w.sep, fb, fc);
-        }
-        normal = capsule_a ? w.normal : -w.normal;
+        if (sep <= accepted) sink.add(pa, pb, sep, fa, fb);
         return MR_STEP_SUCCESS;
     }
     if (cls == MR_COLLISION_PAIR_BOX_BOX) {
         const float3 cd = B.c - A.c;
+        const BoxAxes aa{box_axis(A, 0), box_axis(A, 1), box_axis(A, 2)}, ba{box_axis(B, 0), box_axis(B, 1), box_axis(B, 2)};
         float best_sep = -INFINITY;
         float3 best_n = coincident_normal(ia, ib);
         int best_axis = 0;
@@ -1170,12 +1217,13 @@ __device__ unsigned narrowphase(const Collider& A, const Collider& B, int cls, u
         // (parallel-edge) cross axis shifts the later indices, and the
         // index names the face feature (128 + index).
         int index = -1;
+#pragma unroll 1
         for (int k = 0; k < 15; ++k) {
             float3 axis;
-            if (k < 3) axis = box_axis(A, k);
-            else if (k < 6) axis = box_axis(B, k - 3);
+            if (k < 3) axis = aa[k];
+            else if (k < 6) axis = ba[k - 3];
             else {
-                const float3 cr = cross3(box_axis(A, (k - 6) / 3), box_axis(B, (k - 6) % 3));
+                const float3 cr = cross3(aa[(k - 6) / 3], ba[(k - 6) % 3]);
                 const float sq = dot3(cr, cr);
                 if (!(sq > kParallelEdges)) continue;
                 axis = cr * rsqrtf(sq);
@@ -1183,7 +1231,7 @@ __device__ unsigned narrowphase(const Collider& A, const Collider& B, int cls, u
             ++index;
             const float proj = dot3(cd, axis);
             if (proj < 0.0f || (proj == 0.0f && dot3(axis, best_n) < 0.0f)) axis = -axis;
-            const float sep = fabsf(proj) - box_radius(A, axis) - box_radius(B, axis);
+            const float sep = fabsf(proj) - box_radius(A, aa, axis) - box_radius(B, ba, axis);
             if (sep > accepted) {
                 normal = axis;
                 return MR_STEP_SUCCESS;  // separated: no contact
@@ -1196,29 +1244,38 @@ __device__ unsigned narrowphase(const Collider& A, const Collider& B, int cls, u
             }
         }
         normal = best_n;
-        const float near_b = dot3(B.c, best_n) - box_radius(B, best_n);
-        const float far_a = dot3(A.c, best_n) + box_radius(A, best_n);
-        for (int v = 0; v < 8; ++v) {
-            const float3 pa = box_vertex(A, v);
-            if (!inside_inflated(pa, B, accepted)) continue;
-            const float sep = near_b - dot3(pa, best_n);
-            if (sep <= accepted)
-                sink.add(pa, pa + best_n * sep, sep, feature_key(MR_SHAPE_BOX, static_cast<unsigned>(v)),
-                         feature_key(MR_SHAPE_BOX, 128u + static_cast<unsigned>(best_axis)));
-        }
-        for (int v = 0; v < 8; ++v) {
-            const float3 pb = box_vertex(B, v);
-            if (!inside_inflated(pb, A, accepted)) continue;
-            const float sep = dot3(pb, best_n) - far_a;
-            if (sep <= accepted)
-                sink.add(pb - best_n * sep, pb, sep, feature_key(MR_SHAPE_BOX, 128u + static_cast<unsigned>(best_axis)),
-                         feature_key(MR_SHAPE_BOX, static_cast<unsigned>(v)));
-        }
-        if (sink.count == 0) {
-            const float3 pa = box_support(A, best_n);
-            const float3 pb = box_support(B, -best_n);
-            sink.add(pa, pb, dot3(pb - pa, best_n), feature_key(MR_SHAPE_BOX, 256u + static_cast<unsigned>(best_axis)),
-                     feature_key(MR_SHAPE_BOX, 256u + static_cast<unsigned>(best_axis)));
+        const float near_b = dot3(B.c, best_n) - box_radius(B, ba, best_n);
+        const float far_a = dot3(A.c, best_n) + box_radius(A, aa, best_n);
+        // A's vertices inside B, then B's inside A; the supporting points
+        // when there are none.
+#pragma unroll 1
+        for (int v = 0; v < 17; ++v) {
+            float3 pa, pb;
+            float sep;
+            unsigned fa, fb;
+            if (v < 16) {
+                const bool of_a = v < 8;
+                const Collider& own = of_a ? A : B;
+                const Collider& other = of_a ? B : A;
+                const float3 point = box_vertex(own, v & 7);
+                if (!inside_inflated(point, other, accepted)) continue;
+                sep = of_a ? near_b - dot3(point, best_n) : dot3(point, best_n) - far_a;
+                if (!(sep <= accepted)) continue;
+                const float3 opposite = of_a ? point + best_n * sep : point - best_n * sep;
+                pa = of_a ? point : opposite;
+                pb = of_a ? opposite : point;
+                const unsigned vertex = feature_key(MR_SHAPE_BOX, static_cast<unsigned>(v & 7));
+                const unsigned face = feature_key(MR_SHAPE_BOX, 128u + static_cast<unsigned>(best_axis));
+                fa = of_a ? vertex : face;
+                fb = of_a ? face : vertex;
+            } else {
+                if (sink.count != 0) break;
+                pa = box_support(A, best_n);
+                pb = box_support(B, -best_n);
+                sep = dot3(pb - pa, best_n);
+                fa = fb = feature_key(MR_SHAPE_BOX, 256u + static_cast<unsigned>(best_axis));
+            }
+            sink.add(pa, pb, sep, fa, fb);
         }
         return MR_STEP_SUCCESS;
     }
@@ -1233,6 +1290,7 @@ __device__ unsigned narrowphase(const Collider& A, const Collider& B, int cls, u
         return MR_STEP_SUCCESS;
     }
     if (cls == MR_COLLISION_PAIR_CAPSULE_PLANE) {
+#pragma unroll 1
         for (int e = 0; e < 2; ++e) {
             const float3 surface = (e == 0 ? A.e0 : A.e1) - pn * A.radius;
             const float sep = dot3(pn, surface - B.c);
@@ -1242,6 +1300,7 @@ __device__ unsigned narrowphase(const Collider& A, const Collider& B, int cls, u
         return MR_STEP_SUCCESS;
     }
     if (cls == MR_COLLISION_PAIR_BOX_PLANE) {
+#pragma unroll 1
         for (int v = 0; v < 8; ++v) {
             const float3 w = box_vertex(A, v);
             const float sep = dot3(pn, w - B.c);
@@ -1288,30 +1347,67 @@ __device__ unsigned narrowphase(const Collider& A, const Collider& B, int cls, u
 // (buildPersistentWorldManifold): break thresholds, feature-then-proximity
 // matching, greedy reduction to four with the precision-independent tie
 // rule (scores within a relative 1e-5 go to the smaller feature key), then
-// canonical feature order.  `scratch` holds four old records ahead of the
-// raw records, and 16 candidate-id bytes after them.  Returns the point
-// count, or -1 when non-finite.
-__device__ __forceinline__ unsigned long long rkey(const float* r) {
-    return (static_cast<unsigned long long>(static_cast<unsigned>(ai(r[kCdFaS]))) << 32) | static_cast<unsigned>(ai(r[kCdFbS]));
-}
+// canonical feature order.  `scratch` holds the raw records, `old_world`
+// receives the midpoints and separations of the old points; an old point's
+// anchors and features are read from its slot.  A candidate is a nibble of `geo`
+// (0-3: the old point that holds its geometry, 4 + r: raw record r) and one
+// of `inherit` (the old point whose lifetime and impulse it keeps, 15: new).
+// Returns the point count, or -1 when non-finite.
+struct ManifoldCandidates {
+    float* scratch;
+    float* old_world;
+    const float* old_slot;
+    unsigned long long geo, inherit;
+    int count;
 
-__device__ int build_manifold(const SceneModel& M, const float* old_slot, int nraw, float3 raw_normal, float* scratch,
-                              float* out, float3 posA, float4 rotA, float3 posB, float4 rotB) {
-    const float* raw = scratch + 4 * kRecWords;
-    unsigned char* ids = reinterpret_cast<unsigned char*>(scratch + (4 + kRawCap) * kRecWords);
-    if (nraw == 0) {
-        for (int k = 0; k < 56; ++k) out[k] = 0.0f;
-        return 0;
+    __device__ __forceinline__ int geometry(int k) const { return static_cast<int>((geo >> (4 * k)) & 15ull); }
+    __device__ __forceinline__ int source(int k) const { return static_cast<int>((inherit >> (4 * k)) & 15ull); }
+    // Anchors and features (eight words) of geometry id g.
+    __device__ __forceinline__ const float* anchors(int g) const {
+        return g < 4 ? old_slot + 8 + g * 12 : scratch + (g - 4) * kRawWords;
     }
+    // World midpoint and separation (four words).
+    __device__ __forceinline__ float* world(int g) const {
+        return g < 4 ? old_world + g * kOldWords : scratch + (g - 4) * kRawWords + kRwWp;
+    }
+    __device__ __forceinline__ unsigned long long key(int k) const {
+        const float* r = anchors(geometry(k));
+        return (static_cast<unsigned long long>(static_cast<unsigned>(ai(r[kRwFa]))) << 32) | static_cast<unsigned>(ai(r[kRwFb]));
+    }
+    __device__ __forceinline__ void set_geometry(int k, int g) {
+        geo = (geo & ~(15ull << (4 * k))) | (static_cast<unsigned long long>(g) << (4 * k));
+    }
+    __device__ __forceinline__ void push(int g, int from) {
+        geo |= static_cast<unsigned long long>(g) << (4 * count);
+        inherit |= static_cast<unsigned long long>(from) << (4 * count);
+        ++count;
+    }
+    // Candidate `from` moves to place `to` <= from, those between one up.
+    __device__ __forceinline__ void move_down(int from, int to) {
+        auto moved = [&](unsigned long long v) {
+            const unsigned long long x = (v >> (4 * from)) & 15ull;
+            const unsigned long long below = (1ull << (4 * to)) - 1ull;
+            const unsigned long long above = ~((16ull << (4 * from)) - 1ull);
+            const unsigned long long between = ((1ull << (4 * from)) - 1ull) & ~below;
+            return (v & below) | (x << (4 * to)) | ((v & between) << 4) | (v & above);
+        };
+        geo = moved(geo);
+        inherit = moved(inherit);
+    }
+};
+
+__device__ __forceinline__ int build_manifold(const SceneModel& M, const float* old_slot, int nraw, float3 raw_normal, float* scratch,
+                                              float* old_world, float* out, float3 posA, float4 rotA, float3 posB, float4 rotB) {
+#pragma unroll 1
     for (int i = 0; i < nraw; ++i) {
-        const float* r = raw + i * kRecWords;
-        if (!isfinite(r[kCdSepS]) || !finite3(ld3(r + kCdWpS)) || !finite3(ld3(r + kCdLaS)) || !finite3(ld3(r + kCdLbS)))
+        const float* r = scratch + i * kRawWords;
+        if (!isfinite(r[kRwSep]) || !finite3(ld3(r + kRwWp)) || !finite3(ld3(r + kRwLa)) || !finite3(ld3(r + kRwLb)))
             return -1;
     }
     const float3 nw = raw_normal * (1.0f / len3(raw_normal));
     if (!finite3(nw) || dot3(nw, nw) < 0.9999f) return -1;
     const float4 thr = make_float4(M.thresholds[0], M.thresholds[1], M.thresholds[2], M.thresholds[3]);
-    int nc = 0;
+    ManifoldCandidates cd{scratch, old_world, old_slot, 0ull, 0ull, 0};
     bool old_ok = false;
     float3 transported = f3(0.0f, 0.0f, 0.0f);
     float old_age = 0.0f;
@@ -1324,6 +1420,7 @@ __device__ int build_manifold(const SceneModel& M, const float* old_slot, int nr
             const float3 ot = qrot(rotA, ld3(old_slot + 4));
             transported = ot - nw * dot3(ot, nw);
             old_age = old_slot[3];
+#pragma unroll 1
             for (int i = 0; i < old_count; ++i) {
                 const float* op = old_slot + 8 + i * 12;
                 const float3 pa = posA + qrot(rotA, ld3(op));
@@ -1332,70 +1429,66 @@ __device__ int build_manifold(const SceneModel& M, const float* old_slot, int nr
                 const float sep = dot3(delta, nw);
                 const float3 tan = delta - nw * sep;
                 if (sep > thr.x || len3(tan) > thr.y) continue;
-                float* rec = scratch + i * kRecWords;
-                for (int k = 0; k < 8; ++k) rec[k] = op[k];
-                const unsigned life = static_cast<unsigned>(ai(op[8]));
-                rec[kCdLifeS] = af(static_cast<int>(life == 0xffffffffu ? 0xffffffffu : life + 1u));
-                rec[kCdImpS + 0] = op[9];
-                rec[kCdImpS + 1] = op[10];
-                rec[kCdImpS + 2] = op[11];
-                st3(rec + kCdWpS, 0.5f * (pa + pb));
-                rec[kCdSepS] = sep;
-                ids[nc++] = static_cast<unsigned char>((i << 4) | i);
+                float* w = cd.world(i);
+                st3(w, 0.5f * (pa + pb));
+                w[3] = sep;
+                cd.push(i, i);
             }
         }
     }
     const float merge2 = thr.z * thr.z;
+#pragma unroll 1
     for (int r = 0; r < nraw; ++r) {
-        const float* rr = raw + r * kRecWords;
-        const float3 la = ld3(rr + kCdLaS), lb = ld3(rr + kCdLbS);
-        const int fa = ai(rr[kCdFaS]), fb = ai(rr[kCdFbS]);
+        const float* rr = scratch + r * kRawWords;
+        const float3 la = ld3(rr + kRwLa), lb = ld3(rr + kRwLb);
+        const int fa = ai(rr[kRwFa]), fb = ai(rr[kRwFb]);
         int match = -1;
-        for (int k = 0; k < nc && match < 0; ++k) {
-            const float* g = scratch + (ids[k] & 15u) * kRecWords;
-            if (ai(g[kCdFaS]) == fa && ai(g[kCdFbS]) == fb) match = k;
+#pragma unroll 1
+        for (int k = 0; k < cd.count && match < 0; ++k) {
+            const float* g = cd.anchors(cd.geometry(k));
+            if (ai(g[kRwFa]) == fa && ai(g[kRwFb]) == fb) match = k;
         }
-        for (int k = 0; k < nc && match < 0; ++k) {
-            const float* g = scratch + (ids[k] & 15u) * kRecWords;
-            const float3 da = ld3(g + kCdLaS) - la, db = ld3(g + kCdLbS) - lb;
+#pragma unroll 1
+        for (int k = 0; k < cd.count && match < 0; ++k) {
+            const float* g = cd.anchors(cd.geometry(k));
+            const float3 da = ld3(g + kRwLa) - la, db = ld3(g + kRwLb) - lb;
             if (dot3(da, da) + dot3(db, db) <= 2.0f * merge2) match = k;
         }
         if (match < 0) {
-            if (nc >= 4 + kRawCap) return -1;
-            ids[nc++] = static_cast<unsigned char>((15u << 4) | (4u + r));
+            if (cd.count >= 4 + kRawCap) return -1;
+            cd.push(4 + r, 15);
         } else {
-            ids[match] = static_cast<unsigned char>((ids[match] & 0xf0u) | (4u + r));
+            cd.set_geometry(match, 4 + r);
         }
     }
+    int nc = cd.count;
     if (nc > 4) {
+#pragma unroll 1
         for (int i = 1; i < nc; ++i) {
-            const unsigned char val = ids[i];
-            const float* gv = scratch + (val & 15u) * kRecWords;
-            const float sv = gv[kCdSepS];
-            const unsigned long long kv = rkey(gv);
+            const float sv = cd.world(cd.geometry(i))[3];
+            const unsigned long long kv = cd.key(i);
             int d = i;
             while (d > 0) {
-                const float* gp = scratch + (ids[d - 1] & 15u) * kRecWords;
-                const float sp = gp[kCdSepS];
-                if (!(sv < sp || (sv == sp && kv < rkey(gp)))) break;
-                ids[d] = ids[d - 1];
+                const float sp = cd.world(cd.geometry(d - 1))[3];
+                if (!(sv < sp || (sv == sp && kv < cd.key(d - 1)))) break;
                 --d;
             }
-            ids[d] = val;
+            cd.move_down(i, d);
         }
         unsigned selected = 1u;
         unsigned chosen = 0u;
         int chosen_count = 1;
-        const float3 w0 = ld3(scratch + (ids[0] & 15u) * kRecWords + kCdWpS);
+        const float3 w0 = ld3(cd.world(cd.geometry(0)));
         float3 w1 = w0;
+#pragma unroll 1
         for (int stage = 1; stage < 4; ++stage) {
             int best = -1;
             float best_score = -1.0f;
             unsigned long long best_f = ~0ull;
+#pragma unroll 1
             for (int i = 0; i < nc; ++i) {
                 if (selected & (1u << i)) continue;
-                const float* gi = scratch + (ids[i] & 15u) * kRecWords;
-                const float3 wi = ld3(gi + kCdWpS);
+                const float3 wi = ld3(cd.world(cd.geometry(i)));
                 float score;
                 if (stage == 1) {
                     const float3 dl = wi - w0;
@@ -1405,14 +1498,15 @@ __device__ int build_manifold(const SceneModel& M, const float* old_slot, int nr
                     score = fabsf(dot3(cross3(w1 - w0, wi - w0), nw));
                 } else {
                     score = INFINITY;
+#pragma unroll 1
                     for (int k = 0; k < chosen_count; ++k) {
                         const int ck = static_cast<int>((chosen >> (8 * k)) & 0xffu);
-                        const float3 dl = wi - ld3(scratch + (ids[ck] & 15u) * kRecWords + kCdWpS);
+                        const float3 dl = wi - ld3(cd.world(cd.geometry(ck)));
                         const float3 t = dl - nw * dot3(dl, nw);
                         score = fminf(score, dot3(t, t));
                     }
                 }
-                const unsigned long long f = rkey(gi);
+                const unsigned long long f = cd.key(i);
                 const float tol = fmaxf(kTieAbs, kTieRel * fmaxf(fabsf(score), fabsf(best_score)));
                 if (score > best_score + tol || (fabsf(score - best_score) <= tol && f < best_f)) {
                     best = i;
@@ -1424,23 +1518,26 @@ __device__ int build_manifold(const SceneModel& M, const float* old_slot, int nr
                 chosen |= static_cast<unsigned>(best) << (8 * chosen_count);
                 ++chosen_count;
                 selected |= 1u << best;
-                if (stage == 1) w1 = ld3(scratch + (ids[best] & 15u) * kRecWords + kCdWpS);
+                if (stage == 1) w1 = ld3(cd.world(cd.geometry(best)));
             }
         }
-        unsigned packed = 0u;
-        for (int k = 0; k < chosen_count; ++k) packed |= static_cast<unsigned>(ids[(chosen >> (8 * k)) & 0xffu]) << (8 * k);
-        for (int k = 0; k < chosen_count; ++k) ids[k] = static_cast<unsigned char>((packed >> (8 * k)) & 0xffu);
+        unsigned long long geo = 0ull, inherit = 0ull;
+#pragma unroll 1
+        for (int k = 0; k < chosen_count; ++k) {
+            const int c = static_cast<int>((chosen >> (8 * k)) & 0xffu);
+            geo |= static_cast<unsigned long long>(cd.geometry(c)) << (4 * k);
+            inherit |= static_cast<unsigned long long>(cd.source(c)) << (4 * k);
+        }
+        cd.geo = geo;
+        cd.inherit = inherit;
         nc = chosen_count;
     }
+#pragma unroll 1
     for (int i = 1; i < nc; ++i) {
-        const unsigned char val = ids[i];
-        const unsigned long long f = rkey(scratch + (val & 15u) * kRecWords);
+        const unsigned long long f = cd.key(i);
         int d = i;
-        while (d > 0 && f < rkey(scratch + (ids[d - 1] & 15u) * kRecWords)) {
-            ids[d] = ids[d - 1];
-            --d;
-        }
-        ids[d] = val;
+        while (d > 0 && f < cd.key(d - 1)) --d;
+        cd.move_down(i, d);
     }
     float3 tw = transported;
     if (!old_ok || !finite3(tw) || dot3(tw, tw) <= 1.0e-12f) tw = stable_tangent(nw);
@@ -1449,27 +1546,48 @@ __device__ int build_manifold(const SceneModel& M, const float* old_slot, int nr
     out[3] = old_ok ? fminf(old_age + 1.0f, 65535.0f) : 0.0f;
     st3(out + 4, qrotinv(rotA, tw));
     out[7] = af(nc);
+#pragma unroll 1
     for (int i = 0; i < 4; ++i) {
         float* op = out + 8 + i * 12;
         if (i < nc) {
-            const unsigned id = ids[i];
-            const float* g = scratch + (id & 15u) * kRecWords;
+            const float* g = cd.anchors(cd.geometry(i));
             for (int k = 0; k < 8; ++k) op[k] = g[k];
-            if ((id >> 4) == 15u) {
+            const int from = cd.source(i);
+            if (from == 15) {
                 op[8] = af(0);
                 op[9] = op[10] = op[11] = 0.0f;
             } else {
-                const float* hrec = scratch + (id >> 4) * kRecWords;
-                op[8] = hrec[kCdLifeS];
-                op[9] = hrec[kCdImpS + 0];
-                op[10] = hrec[kCdImpS + 1];
-                op[11] = hrec[kCdImpS + 2];
+                const float* h = old_slot + 8 + from * 12;
+                const unsigned life = static_cast<unsigned>(ai(h[8]));
+                op[8] = af(static_cast<int>(life == 0xffffffffu ? 0xffffffffu : life + 1u));
+                op[9] = h[9];
+                op[10] = h[10];
+                op[11] = h[11];
             }
         } else {
             for (int k = 0; k < 12; ++k) op[k] = 0.0f;
         }
     }
     return nc;
+}
+
+// Cost group of a pair class (see kPairGroups).
+template <bool kConvex>
+__device__ __forceinline__ int pair_group(int cls) {
+    if (cls == MR_COLLISION_PAIR_BOX_BOX) return 0;
+    if (kConvex) {
+        if (cls == MR_COLLISION_PAIR_CONVEX) return 1;
+        return cls == MR_COLLISION_PAIR_BOX_PLANE || cls == MR_COLLISION_PAIR_CYLINDER_PLANE ? 2 : 3;
+    }
+    if (cls == MR_COLLISION_PAIR_BOX_PLANE) return 1;
+    return cls == MR_COLLISION_PAIR_SPHERE_PLANE || cls == MR_COLLISION_PAIR_CAPSULE_PLANE ? 2 : 3;
+}
+
+// Most raw contacts of a pair class.
+__device__ __forceinline__ int pair_raws(int cls) {
+    if (cls == MR_COLLISION_PAIR_BOX_BOX || cls == MR_COLLISION_PAIR_BOX_PLANE) return kRawCap;
+    if (cls == MR_COLLISION_PAIR_CONVEX || cls == MR_COLLISION_PAIR_CYLINDER_PLANE) return 5;  // a witness and four patch points
+    return cls == MR_COLLISION_PAIR_CAPSULE_PLANE ? 2 : 1;
 }
 
 // World inverse inertia R diag(inv) R^T, packed (xx, yx, yy, zx, zy, zz).
@@ -1503,22 +1621,74 @@ __device__ void audit_scene(const SceneModel& M, const float* q, const float* v,
     audit_commit(a, rec, reset, lane);
 }
 
-// kComp: compensated sums for positions (across control steps, through
-// p.q_comp) and for the velocity increments of the sweeps.  kConvex: the
-// world has support-mapped (cylinder) pairs.
+// Solver row of one contact: its frame's tangents (the normal stays in
+// shared memory as well), evaluated target and regularisation, friction,
+// relaxation, impulse and block preconditioner.
+struct ContactRow {
+    float3 n, t, bt;
+    float target, reg, mu, relax;
+    float3 lambda;
+    float pre[9];
+};
+// Rows past the first per thread, word-major in the workspace.
+__device__ __forceinline__ void store_row(float* R, int c, const ContactRow& r) {
+    const float w[kRowWords] = {r.n.x, r.n.y, r.n.z, r.t.x, r.t.y, r.t.z, r.bt.x, r.bt.y, r.bt.z, r.target, r.reg, r.mu, r.relax,
+                                r.lambda.x, r.lambda.y, r.lambda.z, r.pre[0], r.pre[1], r.pre[2], r.pre[3], r.pre[4], r.pre[5],
+                                r.pre[6], r.pre[7], r.pre[8]};
+#pragma unroll
+    for (int k = 0; k < kRowWords; ++k) R[k * kSceneContacts + c] = w[k];
+}
+__device__ __forceinline__ void load_row(const float* R, int c, ContactRow& r) {
+    float w[kRowWords];
+#pragma unroll
+    for (int k = 0; k < kRowWords; ++k) w[k] = R[k * kSceneContacts + c];
+    r.n = f3(w[0], w[1], w[2]);
+    r.t = f3(w[3], w[4], w[5]);
+    r.bt = f3(w[6], w[7], w[8]);
+    r.target = w[9];
+    r.reg = w[10];
+    r.mu = w[11];
+    r.relax = w[12];
+    r.lambda = f3(w[13], w[14], w[15]);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) r.pre[k] = w[16 + k];
+}
+__device__ __forceinline__ void store_lambda(float* R, int c, float3 l) {
+    R[13 * kSceneContacts + c] = l.x;
+    R[14 * kSceneContacts + c] = l.y;
+    R[15 * kSceneContacts + c] = l.z;
+}
+
+// One CTA advances work item `item` of environment slot `env` by one control
+// step, with `s` its scene_step_smem_bytes() of shared memory.  Every thread
+// of the CTA calls it; it returns with the CTA synchronised on entry to the
+// commit but not after it.  kComp: compensated sums for positions (across
+// control steps, through p.q_comp) and for the velocity increments of the
+// sweeps.  kConvex: the world has support-mapped pairs.
 //
-// One warp advances work item `item` of environment slot `env` by one
-// control step, with `s` the warp's scene_step_smem_bytes() of shared
-// memory.  Only warp-level synchronisation is used.
+// It is compiled once, out of line: the per-world kernel and the batch call
+// the same body with any number of warps, and no arithmetic depends on that
+// number, so a world's results are the same bits from either.
+//
+// What bounds it: instruction issue (47 % of cycles with one warp per
+// environment at 16 warps per SM, 13 of 32 lanes active) and, before the
+// loops were rolled, instruction fetch -- the 260 KB of an unrolled kernel
+// do not stay in the instruction cache with every warp at its own stage, and
+// the same launches ran 1.3 to 1.5 times longer.  Hence `unroll 1` on every
+// loop whose body is more than a few instructions.  Contact rows in
+// registers, arms and impulses in shared memory and the CTA per environment
+// took 16,384 36-body piles from 9.58 to 6.41 ms per control step against
+// one warp per environment with its records in global memory.
 template <bool kComp, bool kConvex>
-__device__ __forceinline__ void scene_step_item(const SceneParams& p, float* s, int item, int env) {
-    const int lane = threadIdx.x & 31;
+__device__ __noinline__ void scene_step_item(const SceneParams& p, float* s, int item, int env) {
+    const int tid = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
+    const int lane = tid & 31, warp = tid >> 5, warps = nt >> 5;
     const SceneModel& M = *p.model;
     if (p.world_tag != 0u && M.world_tag != p.world_tag) {
         // The record behind p.model is not the world this launch was
         // enqueued for: its body count need not match the caller's buffers,
         // so touch none of them.
-        if (lane == 0) {
+        if (tid == 0) {
             if (p.status_codes) p.status_codes[item] = MR_STEP_UNSUPPORTED;
             if (p.active_contacts) p.active_contacts[item] = 0u;
             atomicAdd(p.stats + 0, 1u);
@@ -1529,18 +1699,26 @@ __device__ __forceinline__ void scene_step_item(const SceneParams& p, float* s, 
     }
     const int nb = M.nb;
     const int nq = nb * 7, nv = nb * 6;
-    float* misc = s + kOffMisc;
+    float* fixed = s + off_fixed(nb);
+    float* misc = fixed + kOffMisc;
+    float* shared_union = s + off_union(nb);
+    const int union_words = dynamic_smem_words() - off_union(nb) - comp_words(nb, kComp);
+    float* pos_comp = shared_union + union_words;  // kComp only
+    float* lin_comp = pos_comp + 3 * nb;
+    float* ang_comp = pos_comp + 6 * nb;
     const float h = M.h;
-    if (lane < 32) misc[lane] = 0.0f;
+    if (tid < 32) misc[tid] = tid == kSmStatus ? af(static_cast<int>(kNoFailure)) : 0.0f;
     const bool reset = p.reset_masks != nullptr && p.reset_masks[item] != 0u;
     const float* srcq = (reset ? p.reset_q : p.q) + static_cast<size_t>(env) * nq;
     const float* srcv = (reset ? p.reset_v : p.v) + static_cast<size_t>(env) * nv;
-    for (int b = lane; b < nb; b += 32) {
-        st3(s + kOffPos + b * 3, ld3(srcq + b * 7));
-        st4(s + kOffQuat + b * 4, ld4(srcq + b * 7 + 3));
-        st3(s + kOffLin + b * 3, ld3(srcv + b * 6));
-        st3(s + kOffAng + b * 3, ld3(srcv + b * 6 + 3));
-        if (kComp) st3(s + kOffPosComp + b * 3, reset ? f3(0.0f, 0.0f, 0.0f) : ld3(p.q_comp + static_cast<size_t>(env) * nq + b * 7));
+#pragma unroll 1
+    for (int b = tid; b < nb; b += nt) {
+        st3(s + off_pos(nb) + b * 3, ld3(srcq + b * 7));
+        st4(s + off_quat(nb) + b * 4, ld4(srcq + b * 7 + 3));
+        st3(s + off_lin(nb) + b * 3, ld3(srcv + b * 6));
+        st3(s + off_ang(nb) + b * 3, ld3(srcv + b * 6 + 3));
+        s[off_im(nb) + b] = M.mass[b].y;
+        if (kComp) st3(pos_comp + b * 3, reset ? f3(0.0f, 0.0f, 0.0f) : ld3(p.q_comp + static_cast<size_t>(env) * nq + b * 7));
     }
     // Manifold table (sorted by pair key); a reset clears it.  Substeps
     // alternate between the two workspace tables; the environment's own
@@ -1551,32 +1729,56 @@ __device__ __forceinline__ void scene_step_item(const SceneParams& p, float* s, 
     int mcount = reset ? 0 : static_cast<int>(p.manifold_count[env]);
     // Shared copies of the current table's pair keys (binary search) and of
     // the next one's, built as the narrowphase writes it.
-    std::uint32_t* keys_cur = reinterpret_cast<std::uint32_t*>(s + kOffKeys);
-    std::uint32_t* keys_next = keys_cur + kSceneManifolds;
-    for (int i = lane; i < mcount; i += 32) keys_cur[i] = static_cast<std::uint32_t>(ai(persistent[i * kSceneSlotWords + 56]));
+    std::uint16_t* keys_cur = reinterpret_cast<std::uint16_t*>(fixed + kOffKeys);
+    std::uint16_t* keys_next = keys_cur + kSceneManifolds;
+#pragma unroll 1
+    for (int i = tid; i < mcount; i += nt) keys_cur[i] = static_cast<std::uint16_t>(min(static_cast<unsigned>(ai(persistent[i * kSceneSlotWords + 56])), 0xffffu));
     const float friction_scale = p.friction_scale[env];
-    __syncwarp();
+    std::uint16_t* cand = reinterpret_cast<std::uint16_t*>(fixed + kOffCand);
+    std::uint16_t* entries = reinterpret_cast<std::uint16_t*>(fixed + kOffCand);
+    std::uint16_t* mfirst = reinterpret_cast<std::uint16_t*>(fixed + kOffFirst);
+    std::uint16_t* mab = reinterpret_cast<std::uint16_t*>(fixed + kOffAb);
+    std::uint16_t* cmap = reinterpret_cast<std::uint16_t*>(fixed + kOffMap);
+    std::uint16_t* cab = reinterpret_cast<std::uint16_t*>(fixed + kOffCab);
+    std::uint8_t* sorted = reinterpret_cast<std::uint8_t*>(fixed + kOffSorted);
+    unsigned* touching = reinterpret_cast<unsigned*>(misc) + kSmTouching;
+    unsigned* mask = reinterpret_cast<unsigned*>(s + off_lo(nb));
+    unsigned* bits = reinterpret_cast<unsigned*>(shared_union);
+    std::uint16_t* scratch_at = reinterpret_cast<std::uint16_t*>(fixed + kOffScratch);
+    int* start = reinterpret_cast<int*>(fixed + kOffLists);
+    float* rows = ws + kWsRows;
+    __syncthreads();
 
+#pragma unroll 1
     for (int sub = 0; sub < p.substeps; ++sub) {
         const bool final_substep = sub + 1 == p.substeps;
+        bool failed = false;
         // Prediction, world inverse inertia, swept bounds.
-        for (int b = lane; b < nb; b += 32) {
+#pragma unroll 1
+        for (int b = tid; b < nb; b += nt) {
             const float4 m = M.mass[b];
-            float3 lin = ld3(s + kOffLin + b * 3), ang = ld3(s + kOffAng + b * 3);
+            float3 lin = ld3(s + off_lin(nb) + b * 3), ang = ld3(s + off_ang(nb) + b * 3);
             lin = expf(-h * m.z) * lin + h * f3(M.gravity[0], M.gravity[1], M.gravity[2]);
             ang = expf(-h * m.w) * ang;
-            if (!finite3(lin) || !finite3(ang)) fail(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(b));
-            st3(s + kOffLin + b * 3, lin);
-            st3(s + kOffAng + b * 3, ang);
-            float4 q = ld4(s + kOffQuat + b * 4);
+            if (!finite3(lin) || !finite3(ang)) {
+                fail(misc, 0u, MR_STEP_NONFINITE_RESULT);
+                failed = true;
+            }
+            st3(s + off_lin(nb) + b * 3, lin);
+            st3(s + off_ang(nb) + b * 3, ang);
+            float4 q = ld4(s + off_quat(nb) + b * 4);
             float4 qn;
             if (!qnormalize(q, qn, true)) {
-                fail(misc, MR_STEP_NONFINITE_INPUT, static_cast<unsigned>(b));
+                fail(misc, 1u, MR_STEP_NONFINITE_INPUT);
+                failed = true;
                 qn = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
             }
-            const float3 c = ld3(s + kOffPos + b * 3);
-            if (!finite3(c)) fail(misc, MR_STEP_NONFINITE_INPUT, static_cast<unsigned>(b));
-            world_inv_inertia(qn, M.inv_inertia[b], s + kOffIiw + b * 6);
+            const float3 c = ld3(s + off_pos(nb) + b * 3);
+            if (!finite3(c)) {
+                fail(misc, 1u, MR_STEP_NONFINITE_INPUT);
+                failed = true;
+            }
+            world_inv_inertia(qn, M.inv_inertia[b], s + off_iiw(nb) + b * 6);
             // Speculative sweep over the substep (Collision.metal:5960-6030).
             const float4 off = M.offsets[b];
             const float3 fc = c + h * lin;
@@ -1589,7 +1791,7 @@ __device__ __forceinline__ void scene_step_item(const SceneParams& p, float* s, 
             const float chord = 2.0f * off.z * fabsf(sinf(0.5f * h * len3(ang)));
             const float envelope = fminf(len3(fc - c) + chord, h * M.speed_envelope);
             const float margin = M.speculative_scale * envelope;
-            s[kOffMargin + b] = margin;
+            s[off_margin(nb) + b] = margin;
             const float4 dm = M.dims[b];
             float3 e0, e1;
             if (M.shape_type[b] == MR_SHAPE_SPHERE) {
@@ -1624,73 +1826,161 @@ __device__ __forceinline__ void scene_step_item(const SceneParams& p, float* s, 
                                  fmaxf(fabsf(lo.z), fabsf(hi.z)) + 1.0f);
             lo = lo - sc * kAabbPadS - f3(margin, margin, margin);
             hi = hi + sc * kAabbPadS + f3(margin, margin, margin);
-            st3(s + kOffLo + b * 3, lo);
-            st3(s + kOffHi + b * 3, hi);
-            st4(s + kOffQuat + b * 4, qn);
+            st3(s + off_lo(nb) + b * 3, lo);
+            st3(s + off_hi(nb) + b * 3, hi);
+            st4(s + off_quat(nb) + b * 4, qn);
         }
-        if (!ok(misc)) break;
+        if (__syncthreads_or(failed)) break;
 
-        // Pair flags over the compiled list, compacted in pair order.
-        std::uint16_t* cand = reinterpret_cast<std::uint16_t*>(s + kOffCand);
-        int ncand = 0;
-        bool overflow = false;
-        for (int base = 0; base < M.np; base += 32) {
-            const int pi = base + lane;
+        // Pair flags over the compiled list, one ballot word per 32 pairs,
+        // then compacted in pair order: each warp sums the words ahead of its
+        // own.
+        const int words = (M.np + 31) >> 5;
+#pragma unroll 1
+        for (int w = warp; w < words; w += warps) {
+            const int pi = w * 32 + lane;
             bool flag = false;
             if (pi < M.np) {
                 const int a = M.pair_a[pi], b = M.pair_b[pi];
-                const float3 la = ld3(s + kOffLo + a * 3), ha = ld3(s + kOffHi + a * 3);
+                const float3 la = ld3(s + off_lo(nb) + a * 3), ha = ld3(s + off_hi(nb) + a * 3);
                 if (b >= nb) {
                     const float3 pn = qrot(M.plane_rotation, f3(0.0f, 1.0f, 0.0f));
                     const float3 n = pn * rsqrtf(dot3(pn, pn));
                     const float3 center = 0.5f * (la + ha), halfx = 0.5f * (ha - la);
-                    const float off = M.offsets[a].x + s[kOffMargin + a];
+                    const float off = M.offsets[a].x + s[off_margin(nb) + a];
                     const float scale = fmaxf(fmaxf(maxabs3(xyz(M.plane_position)), maxabs3(la)),
                                               fmaxf(maxabs3(ha), fmaxf(fabsf(M.plane_offsets.x), fabsf(off))));
                     const float3 an = f3(fabsf(n.x), fabsf(n.y), fabsf(n.z));
                     flag = dot3(n, center - xyz(M.plane_position)) - dot3(an, halfx) <= M.plane_offsets.x + (scale + 1.0f) * kQueryPadS;
                 } else {
-                    const float3 lb = ld3(s + kOffLo + b * 3), hb = ld3(s + kOffHi + b * 3);
+                    const float3 lb = ld3(s + off_lo(nb) + b * 3), hb = ld3(s + off_hi(nb) + b * 3);
                     flag = la.x <= hb.x && lb.x <= ha.x && la.y <= hb.y && lb.y <= ha.y && la.z <= hb.z && lb.z <= ha.z;
                 }
             }
             const unsigned m = __ballot_sync(0xffffffffu, flag);
-            const int at = ncand + __popc(m & ((1u << lane) - 1u));
-            if (flag) {
-                if (at < kSceneCandidates) cand[at] = static_cast<std::uint16_t>(pi);
-                else overflow = true;
-            }
-            ncand += __popc(m);
+            if (lane == 0) bits[w] = m;
         }
-        if (__any_sync(0xffffffffu, overflow)) {
-            if (lane == 0) fail(misc, MR_STEP_PAIR_CAPACITY_OVERFLOW, static_cast<unsigned>(ncand));
-            __syncwarp();
+        if (tid < 4) touching[tid] = 0u;
+        if (tid == 0) misc[kSmRawNow] = af(0);
+        __syncthreads();
+        int ncand = 0;
+#pragma unroll 1
+        for (int w0 = 0; w0 < words; w0 += 32) {
+            const unsigned m = w0 + lane < words ? bits[w0 + lane] : 0u;
+            int incl = __popc(m);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            const int before = ncand + incl - __popc(m);
+#pragma unroll 1
+            for (int w = warp; w < 32 && w0 + w < words; w += warps) {
+                const unsigned mw = __shfl_sync(0xffffffffu, m, w);
+                const int at = __shfl_sync(0xffffffffu, before, w) + __popc(mw & ((1u << lane) - 1u));
+                if (((mw >> lane) & 1u) && at < kSceneCandidates) cand[at] = static_cast<std::uint16_t>((w0 + w) * 32 + lane);
+            }
+            ncand += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (ncand > kSceneCandidates) {
+            if (tid == 0) fail(misc, 0u, MR_STEP_PAIR_CAPACITY_OVERFLOW);
             break;
         }
-        if (lane == 0) misc[kSmCand] = af(max(ai(misc[kSmCand]), ncand));
-        __syncwarp();
+        if (tid == 0) misc[kSmCand] = af(max(ai(misc[kSmCand]), ncand));
+        __syncthreads();
 
-        // Narrowphase + manifolds, 32 candidates at a time.  A pair with raw
-        // contacts always yields a manifold, so its table position is known
-        // before the manifold is built, and it is built in place.
+        // Narrowphase + manifolds, kPairBlock candidates at a time.  A pair
+        // with raw contacts always yields a manifold, so once the block's
+        // pairs with contacts are known so are their table positions (in pair
+        // order), and each manifold is built in place by its pair's lane.
         const float* old_table = cur_table;
         float* new_table = ws + ((sub & 1) ? kWsTable1 : kWsTable0);
-        float* scratch = ws + kWsLanes + lane * kLaneScratch;
-        int ncount = 0, raw_total = 0;
-        bool bad = false, mover = false, unresolved = false;
-        for (int base = 0; base < ncand; base += 32) {
-            const int ci = base + lane;
+        int ncount = 0;
+#pragma unroll 1
+        for (int base = 0, round = 0, block = 0; base < ncand; base += block, ++round) {
+            // Every warp lays out and ranks the block's pairs; warp 0
+            // publishes the order and the scratch offsets.
+            {
+                int group[2], end[2], room[2];
+                int used = 0;
+                bool full = false;
+                block = 0;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int ci = base + j * 32 + lane;
+                    const bool there = ci < ncand && (j == 0 || warps > 1) && !full;
+                    const int cls = there ? M.pair_class[cand[ci]] : -1;
+                    room[j] = there ? pair_raws(cls) * kRawWords + kPairFixed : 0;
+                    end[j] = room[j];
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int t = __shfl_up_sync(0xffffffffu, end[j], o);
+                        if (lane >= o) end[j] += t;
+                    }
+                    end[j] += used;
+                    used = __shfl_sync(0xffffffffu, end[j], 31);
+                    const bool fits = there && end[j] <= union_words;
+                    full = used > union_words;
+                    group[j] = fits ? pair_group<kConvex>(cls) : kPairGroups;
+                    block += __popc(__ballot_sync(0xffffffffu, fits));
+                }
+                int at = 0, place[2] = {0, 0};
+#pragma unroll
+                for (int g = 0; g < kPairGroups; ++g)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const unsigned of_group = __ballot_sync(0xffffffffu, group[j] == g);
+                        if (group[j] == g) place[j] = at + __popc(of_group & ((1u << lane) - 1u));
+                        at += __popc(of_group);
+                    }
+                if (warp == 0) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        if (group[j] < kPairGroups) {
+                            sorted[place[j]] = static_cast<std::uint8_t>(j * 32 + lane);
+                            scratch_at[j * 32 + lane] = static_cast<std::uint16_t>(end[j] - room[j]);
+                        }
+                }
+            }
+            __syncthreads();
+            unsigned* touch = touching + (round & 1) * 2;
+            const int share = min(32, kPairBlock / warps);
+            const int place = warp * share + lane;
+            const bool mine = lane < share && place < block;
+            const int i = mine ? sorted[place] : 0;
+            const int pi = cand[base + i];
+            const int a = M.pair_a[pi], b = M.pair_b[pi];
+            const int cls = M.pair_class[pi];
+            float* scratch = shared_union + (mine ? scratch_at[i] : 0);
+            float* old_world = scratch + pair_raws(cls) * kRawWords;
             int nraw = 0;
-            unsigned key = 0u;
-            const float* old_slot = nullptr;
-            float3 normal = f3(0.0f, 0.0f, 1.0f);
-            float3 posA = f3(0.0f, 0.0f, 0.0f), posB = posA;
-            float4 rotA = make_float4(0.0f, 0.0f, 0.0f, 1.0f), rotB = rotA;
-            if (ci < ncand) {
-                const int pi = cand[ci];
-                const int a = M.pair_a[pi], b = M.pair_b[pi];
-                key = static_cast<unsigned>(a * (kSceneMaxBodies + 1) + b);
+            if (mine) {
+                Collider A, B;
+                load_collider(M, s, a, A);
+                load_collider(M, s, b, B);
+                const float accepted = A.offset + B.offset + (fmaxf(collider_scale(A), collider_scale(B)) + 1.0f) * kQueryPadS;
+                RawSink sink{scratch, 0, A.bpos, B.bpos, A.brot, B.brot};
+                float3 normal = f3(0.0f, 0.0f, 1.0f);
+                if (narrowphase<kConvex>(A, B, cls, static_cast<unsigned>(a), static_cast<unsigned>(b), accepted, sink,
+                                         normal) != MR_STEP_SUCCESS) {
+                    fail(misc, 0u, MR_STEP_DID_NOT_CONVERGE);
+                    failed = true;
+                }
+                nraw = sink.count;
+                if (nraw > 0) {
+                    st3(old_world + 4 * kOldWords, normal);
+                    atomicOr(touch + (i >> 5), 1u << (i & 31));
+                    atomicAdd(reinterpret_cast<int*>(misc) + kSmRawNow, nraw);
+                }
+            }
+            __syncthreads();
+            const unsigned touched[2] = {touch[0], touch[1]};
+            const unsigned below = (1u << (i & 31)) - 1u;
+            const int at = ncount + (i < 32 ? __popc(touched[0] & below) : __popc(touched[0]) + __popc(touched[1] & below));
+            if (nraw > 0 && at < kSceneManifolds) {
+                const unsigned key = static_cast<unsigned>(a * (kSceneMaxBodies + 1) + b);
                 // Old manifold of this pair (keys ascending).
+                const float* old_slot = nullptr;
                 int lo_i = 0, hi_i = mcount - 1;
                 while (lo_i <= hi_i) {
                     const int mid = (lo_i + hi_i) >> 1;
@@ -1699,427 +1989,526 @@ __device__ __forceinline__ void scene_step_item(const SceneParams& p, float* s, 
                     if (mk < key) lo_i = mid + 1;
                     else hi_i = mid - 1;
                 }
-                Collider A, B;
-                load_collider(M, s, a, A);
-                load_collider(M, s, b, B);
-                const float accepted = A.offset + B.offset + (fmaxf(collider_scale(A), collider_scale(B)) + 1.0f) * kQueryPadS;
-                RawSink sink{scratch + 4 * kRecWords, 0, A.bpos, B.bpos, A.brot, B.brot};
-                if (narrowphase<kConvex>(A, B, M.pair_class[pi], static_cast<unsigned>(a), static_cast<unsigned>(b), accepted, sink,
-                                         normal) != MR_STEP_SUCCESS)
-                    unresolved = true;
-                nraw = sink.count;
-                posA = A.bpos;
-                rotA = A.brot;
-                posB = B.bpos;
-                rotB = B.brot;
-            }
-            raw_total += nraw;
-            const unsigned m = __ballot_sync(0xffffffffu, nraw > 0);
-            const int at = ncount + __popc(m & ((1u << lane) - 1u));
-            if (nraw > 0) {
-                if (at < kSceneManifolds) {
-                    float* dst = new_table + at * kSceneSlotWords;
-                    if (build_manifold(M, old_slot, nraw, normal, scratch, dst, posA, rotA, posB, rotB) <= 0) bad = true;
-                    dst[56] = af(static_cast<int>(key));
-                    keys_next[at] = key;
-                } else {
-                    mover = true;
+                const bool plane_b = b >= nb;
+                const float3 posA = ld3(s + off_pos(nb) + a * 3);
+                const float4 rotA = ld4(s + off_quat(nb) + a * 4);
+                const float3 posB = plane_b ? xyz(M.ground_position) : ld3(s + off_pos(nb) + b * 3);
+                const float4 rotB = plane_b ? M.ground_rotation : ld4(s + off_quat(nb) + b * 4);
+                float* dst = new_table + at * kSceneSlotWords;
+                const int points = build_manifold(M, old_slot, nraw, ld3(old_world + 4 * kOldWords), scratch, old_world, dst, posA, rotA,
+                                                  posB, rotB);
+                if (points <= 0) {
+                    fail(misc, 1u, MR_STEP_NONFINITE_RESULT);
+                    failed = true;
                 }
+                dst[56] = af(static_cast<int>(key));
+                keys_next[at] = static_cast<std::uint16_t>(key);
+                mab[at] = static_cast<std::uint16_t>((a << 8) | b);
+                mfirst[at] = static_cast<std::uint16_t>(max(points, 0));
             }
-            ncount += __popc(m);
+            ncount += __popc(touched[0]) + __popc(touched[1]);
+            // The next block's scratch, order and bit set reuse these words.
+            __syncthreads();
+            if (tid < 2) touch[tid] = 0u;
         }
-        raw_total = __reduce_add_sync(0xffffffffu, raw_total);
-        if (__any_sync(0xffffffffu, unresolved)) {
-            if (lane == 0) fail(misc, MR_STEP_DID_NOT_CONVERGE, 0u);
-            __syncwarp();
-            break;
+        if (ncount > kSceneManifolds) {
+            if (tid == 0) fail(misc, 2u, MR_STEP_MANIFOLD_CAPACITY_OVERFLOW);
+            failed = true;
         }
-        if (__any_sync(0xffffffffu, bad)) {
-            if (lane == 0) fail(misc, MR_STEP_NONFINITE_RESULT, 0u);
-            __syncwarp();
-            break;
-        }
-        if (__any_sync(0xffffffffu, mover)) {
-            if (lane == 0) fail(misc, MR_STEP_MANIFOLD_CAPACITY_OVERFLOW, static_cast<unsigned>(ncount));
-            __syncwarp();
-            break;
-        }
-        __syncwarp();
+        if (__syncthreads_or(failed)) break;
+#pragma unroll 1
+        for (int i = tid; i < 4 * nb; i += nt) mask[i] = 0u;
         cur_table = new_table;
         mcount = ncount;
         float* tab = new_table;
         {
-            std::uint32_t* t = keys_cur;
+            std::uint16_t* t = keys_cur;
             keys_cur = keys_next;
             keys_next = t;
         }
-        if (lane == 0) {
-            misc[kSmManifolds] = af(max(ai(misc[kSmManifolds]), mcount));
-            misc[kSmRaw] = af(max(ai(misc[kSmRaw]), raw_total));
-        }
-        __syncwarp();
-
-        // Contact records in manifold order (lane per manifold).
-        float* C = ws + kWsContacts;
-        std::uint16_t* mfirst = reinterpret_cast<std::uint16_t*>(s + kOffFirst);
+        // First contact of each manifold: every warp scans the point counts
+        // in registers, warp 0 publishes them.
+        int first_of[kSceneManifolds / 32];
         int total = 0;
-        for (int base = 0; base < mcount; base += 32) {
-            const int mi = base + lane;
-            const int cnt = mi < mcount ? ai(tab[mi * kSceneSlotWords + 7]) : 0;
+#pragma unroll
+        for (int j = 0; j < kSceneManifolds / 32; ++j) {
+            const int mi = j * 32 + lane;
+            const int cnt = mi < mcount ? mfirst[mi] : 0;
             int incl = cnt;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int t = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += t;
             }
-            const int first = total + incl - cnt;
+            first_of[j] = total + incl - cnt;
             total += __shfl_sync(0xffffffffu, incl, 31);
-            if (mi < mcount) mfirst[mi] = static_cast<std::uint16_t>(min(first, kSceneContacts));
-            if (cnt > 0 && first + cnt <= kSceneContacts) {
-                const float* slot = tab + mi * kSceneSlotWords;
-                const unsigned key = static_cast<unsigned>(ai(slot[56]));
-                const int a = static_cast<int>(key / (kSceneMaxBodies + 1)), b = static_cast<int>(key % (kSceneMaxBodies + 1));
-                const bool plane_b = b >= nb;
-                const float3 posA = ld3(s + kOffPos + a * 3);
-                const float4 rotA = ld4(s + kOffQuat + a * 4);
-                const float3 posB = plane_b ? xyz(M.ground_position) : ld3(s + kOffPos + b * 3);
-                const float4 rotB = plane_b ? M.ground_rotation : ld4(s + kOffQuat + b * 4);
-                float3 nw = qrot(rotA, ld3(slot));
-                nw = nw * (1.0f / len3(nw));
-                float3 tw = qrot(rotA, ld3(slot + 4));
-                tw = tw - nw * dot3(tw, nw);
-                tw = dot3(tw, tw) > 1.0e-12f ? tw * (1.0f / len3(tw)) : stable_tangent(nw);
-                const float3 bw = cross3(nw, tw);
-                const int ma = M.material[a], mb = plane_b ? M.plane_material : M.material[b];
-                const float4 fa = M.material_friction[ma], fb = M.material_friction[mb];
-                const float mu_s = sqrtf(fmaxf(0.0f, fa.x * fb.x)) * friction_scale;
-                const float mu_d = sqrtf(fmaxf(0.0f, fa.y * fb.y)) * friction_scale;
-                const float4 ra = M.material_response[ma], rb = M.material_response[mb];
-                const float rest = M.offsets[a].y + (plane_b ? M.plane_offsets.y : M.offsets[b].y);
-                for (int i = 0; i < cnt; ++i) {
-                    const float* op = slot + 8 + i * 12;
-                    const Rec c = rec(C, first + i);
-                    const float3 pa = posA + qrot(rotA, ld3(op));
-                    const float3 pb = posB + qrot(rotB, ld3(op + 3));
-                    const float3 pw = 0.5f * (pa + pb);
-                    const float sep = dot3(pb - pa, nw) - rest;
-                    c[kScA] = af(a);
-                    c[kScB] = af(plane_b ? -1 : b);
-                    c.set3(kScRa, pw - posA);
-                    c.set3(kScRb, pw - posB);
-                    c.set3(kScN, nw);
-                    c.set3(kScT, tw);
-                    c.set3(kScBt, bw);
-                    const bool new_impact = static_cast<unsigned>(ai(op[8])) == 0u;
-                    c[kScFlags] = af(new_impact ? 1 : 0);
-                    c[kScSlot] = af(mi * 4 + i);
-                    c[kScLambda + 0] = op[9];
-                    c[kScLambda + 1] = op[10];
-                    c[kScLambda + 2] = op[11];
-                    c[kScTarget + 0] = sep > 0.0f ? -sep / h : 0.0f;
-                    c[kScTarget + 1] = 0.0f;
-                    c[kScTarget + 2] = 0.0f;
-                    c[kScReg] = fmaxf((ra.z + rb.z) / (h * h) + (ra.w + rb.w) / h, 0.0f);
-                    c[kScMu] = mu_s;
-                    c[kScRelax] = fminf(fmaxf(fmaxf(ra.x, rb.x), 0.0f), 1.0f);  // restitution until evaluated
-                    c[kScDelta + 0] = fmaxf(ra.y, rb.y);                          // restitution threshold
-                    c[kScDelta + 1] = mu_d;
-                    c[kScDelta + 2] = sep;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            misc[kSmManifolds] = af(max(ai(misc[kSmManifolds]), mcount));
+            misc[kSmRaw] = af(max(ai(misc[kSmRaw]), ai(misc[kSmRawNow])));
+            if (total > kSceneContacts) fail(misc, 0u, MR_STEP_CONTACT_CAPACITY_OVERFLOW);
+        }
+        if (total > kSceneContacts) break;
+        if (warp == 0) {
+#pragma unroll
+            for (int j = 0; j < kSceneManifolds / 32; ++j) {
+                const int mi = j * 32 + lane;
+                if (mi < mcount) mfirst[mi] = static_cast<std::uint16_t>(first_of[j]);
+            }
+            if (lane == 0) {
+                mfirst[mcount] = static_cast<std::uint16_t>(total);
+                misc[kSmContacts] = af(total);
+            }
+        }
+        __syncthreads();
+        // Contacts of each manifold and manifolds of each body.
+#pragma unroll 1
+        for (int mi = tid; mi < mcount; mi += nt) {
+            const int a = mab[mi] >> 8, b = mab[mi] & 0xff;
+            atomicOr(mask + 4 * a + (mi >> 5), 1u << (mi & 31));
+            if (b < nb) atomicOr(mask + 4 * b + (mi >> 5), 1u << (mi & 31));
+            const int first = mfirst[mi], cnt = mfirst[mi + 1] - first;
+#pragma unroll 1
+            for (int i = 0; i < cnt; ++i) {
+                cmap[first + i] = static_cast<std::uint16_t>(mi * 4 + i);
+                cab[first + i] = mab[mi];
+            }
+        }
+        __syncthreads();
+        // Per-body contact list bounds (ascending contact index).
+        if (warp == 0) {
+            int at = 0;
+#pragma unroll 1
+            for (int b0 = 0; b0 < nb; b0 += 32) {
+                const int b = b0 + lane;
+                int cnt = 0;
+                if (b < nb)
+#pragma unroll 1
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll 1
+                        for (unsigned m = mask[4 * b + j]; m != 0u; m &= m - 1u) {
+                            const int mi = j * 32 + __ffs(m) - 1;
+                            cnt += mfirst[mi + 1] - mfirst[mi];
+                        }
+                int incl = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                if (b < nb) start[b] = at + incl - cnt;
+                at += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (lane == 0) start[nb] = at;
+        }
+        // Contact geometry (lane per contact): normal and arms.
+        float* arrays = total * kContactArrays <= union_words ? shared_union : ws + kWsArrays;
+        float* cn = arrays;  // normals, then impulse changes
+        float* cra = arrays + 3 * total;
+        float* crb = arrays + 6 * total;
+#pragma unroll 1
+        for (int c = tid; c < total; c += nt) {
+            const int mi = cmap[c] >> 2;
+            const float* slot = tab + mi * kSceneSlotWords;
+            const float* op = slot + 8 + (cmap[c] & 3) * 12;
+            const int a = cab[c] >> 8, b = cab[c] & 0xff;
+            const bool plane_b = b >= nb;
+            const float3 posA = ld3(s + off_pos(nb) + a * 3);
+            const float4 rotA = ld4(s + off_quat(nb) + a * 4);
+            const float3 posB = plane_b ? xyz(M.ground_position) : ld3(s + off_pos(nb) + b * 3);
+            const float4 rotB = plane_b ? M.ground_rotation : ld4(s + off_quat(nb) + b * 4);
+            float3 nw = qrot(rotA, ld3(slot));
+            nw = nw * (1.0f / len3(nw));
+            const float3 pa = posA + qrot(rotA, ld3(op));
+            const float3 pb = posB + qrot(rotB, ld3(op + 3));
+            const float3 pw = 0.5f * (pa + pb);
+            st3(cn + c * 3, nw);
+            st3(cra + c * 3, pw - posA);
+            st3(crb + c * 3, pw - posB);
+        }
+        __syncthreads();
+        // Per-body contact lists (side bit 1 = B), walked manifold by
+        // manifold: a manifold's contacts are contiguous.
+#pragma unroll 1
+        for (int b = tid; b < nb; b += nt) {
+            int at = start[b];
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j)
+#pragma unroll 1
+                for (unsigned m = mask[4 * b + j]; m != 0u; m &= m - 1u) {
+                    const int mi = j * 32 + __ffs(m) - 1;
+                    const int side = (mab[mi] >> 8) == b ? 0 : 1;
+#pragma unroll 1
+                    for (int c = mfirst[mi]; c < mfirst[mi + 1]; ++c) entries[at++] = static_cast<std::uint16_t>((c << 1) | side);
+                }
+        }
+        // Islands of dynamic bodies joined by contacts: labels start as the
+        // body's own index and every manifold and body lowers them until
+        // none changes, so a label ends as its island's smallest body.  The
+        // solve treats all contacts of an environment together (islands do
+        // not interact in a Jacobi sweep); islands are a diagnostic, counted
+        // on the final substep.
+        if (final_substep) {
+            int* label = reinterpret_cast<int*>(keys_next);  // the previous table's keys are dead by now
+#pragma unroll 1
+            for (int b = tid; b < nb; b += nt) label[b] = b;
+            bool changed = true;
+            while (__syncthreads_or(changed)) {
+                changed = false;
+#pragma unroll 1
+                for (int mi = tid; mi < mcount; mi += nt) {
+                    const int a = mab[mi] >> 8, b = mab[mi] & 0xff;
+                    if (b >= nb) continue;
+                    const int la = label[a], lb = label[b];
+                    if (la != lb) {
+                        atomicMin(label + max(la, lb), min(la, lb));
+                        atomicMin(label + (la > lb ? a : b), min(la, lb));
+                        changed = true;
+                    }
+                }
+                __syncthreads();
+#pragma unroll 1
+                for (int b = tid; b < nb; b += nt) {
+                    const int l = label[label[b]];
+                    if (l != label[b]) {
+                        atomicMin(label + b, l);
+                        changed = true;
+                    }
                 }
             }
-        }
-        if (total > kSceneContacts) {
-            if (lane == 0) fail(misc, MR_STEP_CONTACT_CAPACITY_OVERFLOW, static_cast<unsigned>(total));
-            __syncwarp();
-            break;
-        }
-        if (lane == 0) {
-            misc[kSmContacts] = af(total);
-            mfirst[mcount] = static_cast<std::uint16_t>(total);
-        }
-        __syncwarp();
-
-        // Per-body contact lists (ascending contact index; side bit 1 = B),
-        // walked manifold by manifold: a manifold's contacts are contiguous.
-        int* start = reinterpret_cast<int*>(s + kOffLists);
-        int* fill = start + kSceneMaxBodies + 1;
-        std::uint16_t* entries = reinterpret_cast<std::uint16_t*>(s + kOffEntries);
-        for (int b = lane; b < nb; b += 32) {
-            int cnt = 0;
-            for (int mi = 0; mi < mcount; ++mi) {
-                const unsigned k = keys_cur[mi];
-                if (static_cast<int>(k / (kSceneMaxBodies + 1)) == b || static_cast<int>(k % (kSceneMaxBodies + 1)) == b)
-                    cnt += mfirst[mi + 1] - mfirst[mi];
-            }
-            fill[b] = cnt;
-        }
-        __syncwarp();
-        if (lane == 0) {
-            int acc = 0;
-            for (int b = 0; b < nb; ++b) { start[b] = acc; acc += fill[b]; }
-            start[nb] = acc;
-        }
-        __syncwarp();
-        for (int b = lane; b < nb; b += 32) {
-            int at = start[b];
-            for (int mi = 0; mi < mcount; ++mi) {
-                const unsigned k = keys_cur[mi];
-                const int side = static_cast<int>(k / (kSceneMaxBodies + 1)) == b ? 0
-                                 : (static_cast<int>(k % (kSceneMaxBodies + 1)) == b ? 1 : -1);
-                if (side < 0) continue;
-                for (int c = mfirst[mi]; c < mfirst[mi + 1]; ++c) entries[at++] = static_cast<std::uint16_t>((c << 1) | side);
+            if (warp == 0) {
+                // A body is in an island when a manifold touches it; islands
+                // are numbered by their smallest body.
+                int islands = 0;
+                unsigned roots[kSceneMaxBodies / 32];
+#pragma unroll
+                for (int j = 0; j < kSceneMaxBodies / 32; ++j) {
+                    const int b = j * 32 + lane;
+                    const bool in = b < nb && (mask[4 * b] | mask[4 * b + 1] | mask[4 * b + 2] | mask[4 * b + 3]) != 0u;
+                    roots[j] = __ballot_sync(0xffffffffu, in && label[b] == b);
+                    islands += __popc(roots[j]);
+                }
+                if (p.island_labels) {
+                    std::uint8_t* labels = p.island_labels + static_cast<size_t>(env) * kSceneMaxBodies;
+#pragma unroll
+                    for (int j = 0; j < kSceneMaxBodies / 32; ++j) {
+                        const int b = j * 32 + lane;
+                        if (b >= nb) continue;
+                        const int r = label[b];
+                        const bool in = (roots[r >> 5] >> (r & 31)) & 1u;
+                        int number = __popc(roots[r >> 5] & ((1u << (r & 31)) - 1u));
+                        if (r >= 32) number += __popc(roots[0]);
+                        labels[b] = in ? static_cast<std::uint8_t>(number) : 0xffu;
+                    }
+                }
+                if (lane == 0) misc[kSmIslands] = af(max(ai(misc[kSmIslands]), islands));
             }
         }
-        __syncwarp();
+        __syncthreads();
 
         // ConstraintIR evaluation at the predicted velocities, blocks,
         // preconditioners, relaxation and warm start (lane per contact).
         auto point_velocity = [&](int body, float3 r) {
-            if (body < 0) return f3(0.0f, 0.0f, 0.0f);
-            return ld3(s + kOffLin + body * 3) + cross3(ld3(s + kOffAng + body * 3), r);
+            if (body >= nb) return f3(0.0f, 0.0f, 0.0f);
+            return ld3(s + off_lin(nb) + body * 3) + cross3(ld3(s + off_ang(nb) + body * 3), r);
         };
-        for (int c = lane; c < total; c += 32) {
-            const Rec cr = rec(C, c);
-            const int a = ai(cr[kScA]), b = ai(cr[kScB]);
-            const float3 ra = cr.v3(kScRa), rb = cr.v3(kScRb);
+        ContactRow own[kOwnRows];
+#pragma unroll 1
+        for (int c = tid; c < total; c += nt) {
+            const int mi = cmap[c] >> 2;
+            const float* slot = tab + mi * kSceneSlotWords;
+            const float* op = slot + 8 + (cmap[c] & 3) * 12;
+            const int a = cab[c] >> 8, b = cab[c] & 0xff;
+            const bool plane_b = b >= nb;
+            ContactRow row;
+            row.n = ld3(cn + c * 3);
+            const float3 posA = ld3(s + off_pos(nb) + a * 3);
+            const float4 rotA = ld4(s + off_quat(nb) + a * 4);
+            const float3 posB = plane_b ? xyz(M.ground_position) : ld3(s + off_pos(nb) + b * 3);
+            const float4 rotB = plane_b ? M.ground_rotation : ld4(s + off_quat(nb) + b * 4);
+            const float3 gap = posB + qrot(rotB, ld3(op + 3)) - (posA + qrot(rotA, ld3(op)));
+            const float sep = dot3(gap, row.n) - (M.offsets[a].y + (plane_b ? M.plane_offsets.y : M.offsets[b].y));
+            float3 tw = qrot(rotA, ld3(slot + 4));
+            tw = tw - row.n * dot3(tw, row.n);
+            row.t = dot3(tw, tw) > 1.0e-12f ? tw * (1.0f / len3(tw)) : stable_tangent(row.n);
+            row.bt = cross3(row.n, row.t);
+            const int ma = M.material[a], mb = plane_b ? M.plane_material : M.material[b];
+            const float4 fra = M.material_friction[ma], frb = M.material_friction[mb];
+            const float mu_s = sqrtf(fmaxf(0.0f, fra.x * frb.x)) * friction_scale;
+            const float mu_d = sqrtf(fmaxf(0.0f, fra.y * frb.y)) * friction_scale;
+            const float4 rsa = M.material_response[ma], rsb = M.material_response[mb];
+            const bool new_impact = static_cast<unsigned>(ai(op[8])) == 0u;
+            row.target = sep > 0.0f ? -sep / h : 0.0f;
+            row.reg = fmaxf((rsa.z + rsb.z) / (h * h) + (rsa.w + rsb.w) / h, 0.0f);
+            row.mu = mu_s;
+            const float restitution = fminf(fmaxf(fmaxf(rsa.x, rsb.x), 0.0f), 1.0f);
+            const float threshold = fmaxf(rsa.y, rsb.y);
+            const float3 ra = ld3(cra + c * 3), rb = ld3(crb + c * 3);
             const float3 dv = point_velocity(b, rb) - point_velocity(a, ra);
-            const float3 dirs[3] = {cr.v3(kScN), cr.v3(kScT), cr.v3(kScBt)};
+            const float3 dirs[3] = {row.n, row.t, row.bt};
             const float rel[3] = {dot3(dv, dirs[0]), dot3(dv, dirs[1]), dot3(dv, dirs[2])};
-            const float sep = cr[kScDelta + 2];
             const float tau_c = 2.0f * h;
             const float err = fminf(sep + M.slop, 0.0f);
             const float ratio = h / tau_c;
             float stab = -h * err / (tau_c * tau_c * (1.0f + 2.0f * ratio + ratio * ratio));
             stab = fminf(fmaxf(stab, 0.0f), M.max_depenetration);
-            if (ai(cr[kScFlags]) & 1) {
-                const float incoming = rel[0] - cr[kScTarget + 0];
-                if (incoming < -cr[kScDelta + 0]) stab = fmaxf(stab, -cr[kScRelax] * incoming);
+            if (new_impact) {
+                const float incoming = rel[0] - row.target;
+                if (incoming < -threshold) stab = fmaxf(stab, -restitution * incoming);
             }
-            cr[kScTarget + 0] += stab;
+            row.target += stab;
             const float slip = sqrtf(rel[1] * rel[1] + rel[2] * rel[2]);
-            if (!(slip <= 1.0e-3f)) cr[kScMu] = cr[kScDelta + 1];
+            if (!(slip <= 1.0e-3f)) row.mu = mu_d;
             // W = sum over dynamic sides of m^-1 d_i.d_j + (r x d_i)^T I^-1 (r x d_j).
             float W[3][3];
             for (int i = 0; i < 3; ++i)
                 for (int j = 0; j < 3; ++j) W[i][j] = 0.0f;
+#pragma unroll 1
             for (int side = 0; side < 2; ++side) {
                 const int body = side ? b : a;
-                if (body < 0) continue;
+                if (body >= nb) continue;
                 const float3 r = side ? rb : ra;
-                const float im = M.mass[body].y;
-                const float* S = s + kOffIiw + body * 6;
+                const float im = s[off_im(nb) + body];
+                const float* S = s + off_iiw(nb) + body * 6;
                 float3 rd[3], ird[3];
                 for (int i = 0; i < 3; ++i) { rd[i] = cross3(r, dirs[i]); ird[i] = sym3_mul(S, rd[i]); }
                 for (int i = 0; i < 3; ++i)
                     for (int j = 0; j < 3; ++j) W[i][j] += im * dot3(dirs[i], dirs[j]) + dot3(rd[i], ird[j]);
             }
-            // Row sum of normal couplings over contacts sharing a body.
+            // Row sum of normal couplings over contacts sharing a body: a
+            // contact's list entry names its side, so only contacts of the
+            // same two bodies have a second term.
             float rowsum = 0.0f;
-            const float3 n_i = dirs[0];
+            const float3 rna = cross3(ra, row.n), rnb = cross3(rb, row.n);
+            const float3 ja = sym3_mul(s + off_iiw(nb) + a * 6, rna);
+            const float3 jb = plane_b ? f3(0.0f, 0.0f, 0.0f) : sym3_mul(s + off_iiw(nb) + b * 6, rnb);
+            const float ima = s[off_im(nb) + a], imb = plane_b ? 0.0f : s[off_im(nb) + b];
+#pragma unroll 1
             for (int side = 0; side < 2; ++side) {
                 const int body = side ? b : a;
-                if (body < 0) continue;
+                if (body >= nb) continue;
+#pragma unroll 1
                 for (int k = start[body]; k < start[body + 1]; ++k) {
-                    const int cj = entries[k] >> 1, sj = entries[k] & 1;
-                    const Rec crj = rec(C, cj);
-                    const int oa = ai(crj[kScA]), ob = ai(crj[kScB]);
+                    const int cj = entries[k] >> 1;
+                    const bool at_b = entries[k] & 1;  // `body` is cj's second
+                    const int oa = cab[cj] >> 8, ob = cab[cj] & 0xff;
                     // Skip on the second body when the first one already counted j.
-                    if (side == 1 && (oa == a || ob == a) && a >= 0) continue;
-                    float w = 0.0f;
-                    for (int t = 0; t < 2; ++t) {
-                        const int bi = t ? b : a;
-                        if (bi < 0) continue;
-                        const int tj = (oa == bi) ? 0 : ((ob == bi) ? 1 : -1);
-                        if (tj < 0) continue;
-                        const float si = t ? 1.0f : -1.0f, sjn = tj ? 1.0f : -1.0f;
-                        const float3 ri = t ? rb : ra, rj = crj.v3(tj ? kScRb : kScRa);
-                        const float3 n_j = crj.v3(kScN);
-                        const float3 rni = cross3(ri, n_i), rnj = cross3(rj, n_j);
-                        w += si * sjn * (M.mass[bi].y * dot3(n_i, n_j) + dot3(rni, sym3_mul(s + kOffIiw + bi * 6, rnj)));
-                    }
-                    (void)sj;
+                    if (side == 1 && (oa == a || ob == a)) continue;
+                    const float3 n_j = ld3(cn + cj * 3);
+                    const float nn = dot3(row.n, n_j);
+                    float w = (side ? imb : ima) * nn + dot3(side ? jb : ja, cross3(ld3((at_b ? crb : cra) + cj * 3), n_j));
+                    if (at_b != (side != 0)) w = -w;
+                    // The other body of both (pairs are ordered: same pair).
+                    if (side == 0 && !plane_b && oa == a && ob == b) w += imb * nn + dot3(jb, cross3(ld3(crb + cj * 3), n_j));
                     rowsum += fabsf(w);
                 }
             }
-            const float reg[3] = {cr[kScReg], 0.0f, 0.0f};
+            const float reg[3] = {row.reg, 0.0f, 0.0f};
             const float diag = fabsf(W[0][0]) + reg[0];
             for (int i = 0; i < 3; ++i) W[i][i] += reg[i];
             float inv[3][3];
             if (!invert3x3_reg(W, inv)) {
-                fail(misc, MR_STEP_FACTORIZATION_FAILED, static_cast<unsigned>(c));
-            } else {
+                fail(misc, 0u, MR_STEP_FACTORIZATION_FAILED);
+                failed = true;
                 for (int i = 0; i < 3; ++i)
-                    for (int j = 0; j < 3; ++j) cr[kScPre + i * 3 + j] = inv[i][j];
+                    for (int j = 0; j < 3; ++j) inv[i][j] = 0.0f;
             }
-            cr[kScRelax] = rowsum > fmaxf(diag, kMatrixFloor) ? fminf(fmaxf(diag / rowsum, 1.0f / 32.0f), 1.0f) : 1.0f;
-            const float3 warm = project_cone(cr.v3(kScLambda), cr[kScMu], cr[kScMu]);
-            cr.set3(kScLambda, warm);
-            cr.set3(kScDelta, warm);
-            if (!isfinite(cr[kScTarget])) fail(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(c));
-        }
-        if (!ok(misc)) break;
-        // Islands: min-root union find over dynamic bodies joined by contacts.
-        // The solve treats all contacts of an environment together (islands
-        // do not interact in a Jacobi sweep), so islands are a diagnostic
-        // here, counted on the final substep.
-        if (lane == 0 && total > 0 && final_substep) {
-            int* parent = reinterpret_cast<int*>(keys_next);  // the previous table's keys are dead by now
-            for (int b = 0; b < nb; ++b) parent[b] = b;
-            auto root = [&](int x) { while (parent[x] != x) x = parent[x] = parent[parent[x]]; return x; };
-            unsigned touched[2] = {0u, 0u};
-            for (int c = 0; c < total; ++c) {
-                const int a = ai(rec(C, c)[kScA]), b = ai(rec(C, c)[kScB]);
-                touched[a >> 5] |= 1u << (a & 31);
-                if (b >= 0) {
-                    touched[b >> 5] |= 1u << (b & 31);
-                    const int x = root(a), y = root(b);
-                    if (x != y) parent[max(x, y)] = min(x, y);
+            for (int i = 0; i < 3; ++i)
+                for (int j = 0; j < 3; ++j) row.pre[i * 3 + j] = inv[i][j];
+            row.relax = rowsum > fmaxf(diag, kMatrixFloor) ? fminf(fmaxf(diag / rowsum, 1.0f / 32.0f), 1.0f) : 1.0f;
+            row.lambda = project_cone(f3(op[9], op[10], op[11]), row.mu, row.mu);
+            if (!isfinite(row.target)) {
+                fail(misc, 1u, MR_STEP_NONFINITE_RESULT);
+                failed = true;
+            }
+            bool kept = false;
+#pragma unroll
+            for (int k = 0; k < kOwnRows; ++k)
+                if (c == tid + k * nt) {
+                    own[k] = row;
+                    kept = true;
                 }
-            }
-            int islands = 0;
-            std::uint8_t* labels = p.island_labels ? p.island_labels + static_cast<size_t>(env) * kSceneMaxBodies : nullptr;
-            for (int b = 0; b < nb; ++b) {
-                // A root precedes every member of its set, so its island
-                // index is known before any member asks for it.
-                const int r = root(b);
-                const bool island_root = ((touched[b >> 5] >> (b & 31)) & 1u) && r == b;
-                if (labels) labels[b] = island_root ? static_cast<std::uint8_t>(islands) : (r == b ? 0xffu : labels[r]);
-                if (island_root) ++islands;
-            }
-            misc[kSmIslands] = af(max(ai(misc[kSmIslands]), islands));
-        } else if (lane == 0 && final_substep && p.island_labels) {
-            for (int b = 0; b < nb; ++b) p.island_labels[static_cast<size_t>(env) * kSceneMaxBodies + b] = 0xffu;
+            if (!kept) store_row(rows, c, row);
         }
-        __syncwarp();
-        // Jacobi sweeps (sweep -1 applies the warm start).
         if (kComp) {
-            for (int i = lane; i < nb * 3; i += 32) {
-                s[kOffLinComp + i] = 0.0f;
-                s[kOffAngComp + i] = 0.0f;
+#pragma unroll 1
+            for (int i = tid; i < nb * 3; i += nt) {
+                lin_comp[i] = 0.0f;
+                ang_comp[i] = 0.0f;
             }
         }
+        if (__syncthreads_or(failed)) break;
+        // A contact's row: its thread's registers, or the workspace.
+        auto row_of = [&](int c) {
+            ContactRow row;
+            bool kept = false;
+#pragma unroll
+            for (int k = 0; k < kOwnRows; ++k)
+                if (c == tid + k * nt) {
+                    row = own[k];
+                    kept = true;
+                }
+            if (!kept) load_row(rows, c, row);
+            return row;
+        };
+        // Jacobi sweeps (sweep -1 applies the warm start).
         const int iters = p.velocity_iterations + (final_substep ? p.final_velocity_iterations : 0);
+#pragma unroll 1
         for (int it = -1; it < iters; ++it) {
-            if (it >= 0) {
-                for (int c = lane; c < total; c += 32) {
-                    const Rec cr = rec(C, c);
-                    const int a = ai(cr[kScA]), b = ai(cr[kScB]);
-                    const float3 dv = point_velocity(b, cr.v3(kScRb)) - point_velocity(a, cr.v3(kScRa));
-                    const float3 prev = cr.v3(kScLambda);
-                    const float r0 = cr[kScTarget + 0] - dot3(dv, cr.v3(kScN)) - cr[kScReg] * prev.x;
-                    const float r1 = cr[kScTarget + 1] - dot3(dv, cr.v3(kScT));
-                    const float r2 = cr[kScTarget + 2] - dot3(dv, cr.v3(kScBt));
-                    float3 prop = f3(prev.x + cr[kScPre + 0] * r0 + cr[kScPre + 1] * r1 + cr[kScPre + 2] * r2,
-                                     prev.y + cr[kScPre + 3] * r0 + cr[kScPre + 4] * r1 + cr[kScPre + 5] * r2,
-                                     prev.z + cr[kScPre + 6] * r0 + cr[kScPre + 7] * r1 + cr[kScPre + 8] * r2);
-                    prop = project_cone(prop, cr[kScMu], cr[kScMu]);
-                    const float3 delta = cr[kScRelax] * (prop - prev);
+#pragma unroll 1
+            for (int c = tid; c < total; c += nt) {
+                const ContactRow row = row_of(c);
+                float3 delta = row.lambda;
+                if (it >= 0) {
+                    const int a = cab[c] >> 8, b = cab[c] & 0xff;
+                    const float3 dv = point_velocity(b, ld3(crb + c * 3)) - point_velocity(a, ld3(cra + c * 3));
+                    const float3 prev = row.lambda;
+                    const float r0 = row.target - dot3(dv, row.n) - row.reg * prev.x;
+                    const float r1 = 0.0f - dot3(dv, row.t);
+                    const float r2 = 0.0f - dot3(dv, row.bt);
+                    float3 prop = f3(prev.x + row.pre[0] * r0 + row.pre[1] * r1 + row.pre[2] * r2,
+                                     prev.y + row.pre[3] * r0 + row.pre[4] * r1 + row.pre[5] * r2,
+                                     prev.z + row.pre[6] * r0 + row.pre[7] * r1 + row.pre[8] * r2);
+                    prop = project_cone(prop, row.mu, row.mu);
+                    delta = row.relax * (prop - prev);
                     const float3 next = prev + delta;
                     if (!finite3(next) || !finite3(delta)) {
-                        fail(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(c));
-                        cr.set3(kScDelta, f3(0.0f, 0.0f, 0.0f));
+                        fail(misc, 0u, MR_STEP_NONFINITE_RESULT);
+                        failed = true;
+                        delta = f3(0.0f, 0.0f, 0.0f);
                     } else {
-                        cr.set3(kScLambda, next);
-                        cr.set3(kScDelta, delta);
+                        bool kept = false;
+#pragma unroll
+                        for (int k = 0; k < kOwnRows; ++k)
+                            if (c == tid + k * nt) {
+                                own[k].lambda = next;
+                                kept = true;
+                            }
+                        if (!kept) store_lambda(rows, c, next);
                     }
                 }
-                __syncwarp();
+                st3(cn + c * 3, row.n * delta.x + row.t * delta.y + row.bt * delta.z);
             }
-            for (int b = lane; b < nb; b += 32) {
+            __syncthreads();
+#pragma unroll 1
+            for (int b = tid; b < nb; b += nt) {
                 float3 dl = f3(0.0f, 0.0f, 0.0f), dw = f3(0.0f, 0.0f, 0.0f);
-                for (int k = start[b]; k < start[b + 1]; ++k) {
+                const int end = start[b + 1];
+#pragma unroll 2
+                for (int k = start[b]; k < end; ++k) {
                     const int c = entries[k] >> 1, side = entries[k] & 1;
-                    const Rec cr = rec(C, c);
-                    const float3 d = cr.v3(kScDelta);
-                    const float3 imp = cr.v3(kScN) * d.x + cr.v3(kScT) * d.y + cr.v3(kScBt) * d.z;
+                    const float3 imp = ld3(cn + c * 3);
                     const float3 f = side ? imp : -imp;
                     dl = dl + f;
-                    dw = dw + cross3(cr.v3(side ? kScRb : kScRa), f);
+                    dw = dw + cross3(ld3((side ? crb : cra) + c * 3), f);
                 }
-                const float im = M.mass[b].y;
+                const float im = s[off_im(nb) + b];
                 if (kComp) {
-                    st3(s + kOffLin + b * 3, kahan_madd3(ld3(s + kOffLin + b * 3), im, dl, s + kOffLinComp + b * 3));
-                    st3(s + kOffAng + b * 3,
-                        kahan_madd3(ld3(s + kOffAng + b * 3), 1.0f, sym3_mul(s + kOffIiw + b * 6, dw), s + kOffAngComp + b * 3));
+                    st3(s + off_lin(nb) + b * 3, kahan_madd3(ld3(s + off_lin(nb) + b * 3), im, dl, lin_comp + b * 3));
+                    st3(s + off_ang(nb) + b * 3,
+                        kahan_madd3(ld3(s + off_ang(nb) + b * 3), 1.0f, sym3_mul(s + off_iiw(nb) + b * 6, dw), ang_comp + b * 3));
                 } else {
-                    st3(s + kOffLin + b * 3, ld3(s + kOffLin + b * 3) + im * dl);
-                    st3(s + kOffAng + b * 3, ld3(s + kOffAng + b * 3) + sym3_mul(s + kOffIiw + b * 6, dw));
+                    st3(s + off_lin(nb) + b * 3, ld3(s + off_lin(nb) + b * 3) + im * dl);
+                    st3(s + off_ang(nb) + b * 3, ld3(s + off_ang(nb) + b * 3) + sym3_mul(s + off_iiw(nb) + b * 6, dw));
                 }
             }
-            __syncwarp();
+            __syncthreads();
         }
-        if (!ok(misc)) break;
+        if (__syncthreads_or(failed)) break;
         // Impulses back into the manifold points.
-        for (int c = lane; c < total; c += 32) {
-            const Rec cr = rec(C, c);
-            const int slot = ai(cr[kScSlot]);
-            float* op = tab + (slot >> 2) * kSceneSlotWords + 8 + (slot & 3) * 12;
-            op[9] = cr[kScLambda + 0];
-            op[10] = cr[kScLambda + 1];
-            op[11] = cr[kScLambda + 2];
+#pragma unroll 1
+        for (int c = tid; c < total; c += nt) {
+            const float3 lambda = row_of(c).lambda;
+            const int slot = cmap[c];
+            st3(tab + (slot >> 2) * kSceneSlotWords + 8 + (slot & 3) * 12 + 9, lambda);
         }
         // Speed clamps and integration (exponential map of the orientation).
-        for (int b = lane; b < nb; b += 32) {
-            float3 lin = ld3(s + kOffLin + b * 3), ang = ld3(s + kOffAng + b * 3);
+#pragma unroll 1
+        for (int b = tid; b < nb; b += nt) {
+            float3 lin = ld3(s + off_lin(nb) + b * 3), ang = ld3(s + off_ang(nb) + b * 3);
             const float vmax = M.inv_inertia[b].w, wmax = M.offsets[b].w;
-            const float ls = len3(lin), ws = len3(ang);
+            const float ls = len3(lin), ws_ = len3(ang);
             if (vmax > 0.0f && ls > vmax) lin = lin * (vmax / ls);
-            if (wmax > 0.0f && ws > wmax) ang = ang * (wmax / ws);
-            const float3 c = kComp ? kahan_madd3(ld3(s + kOffPos + b * 3), h, lin, s + kOffPosComp + b * 3)
-                                   : ld3(s + kOffPos + b * 3) + h * lin;
-            float4 q = qmul(so3_increment(h * ang, false), ld4(s + kOffQuat + b * 4));
+            if (wmax > 0.0f && ws_ > wmax) ang = ang * (wmax / ws_);
+            const float3 c = kComp ? kahan_madd3(ld3(s + off_pos(nb) + b * 3), h, lin, pos_comp + b * 3)
+                                   : ld3(s + off_pos(nb) + b * 3) + h * lin;
+            float4 q = qmul(so3_increment(h * ang, false), ld4(s + off_quat(nb) + b * 4));
             const float qq = qdot(q, q);
             if (!finite4(q) || !(qq > 1.0e-12f) || !finite3(c) || !finite3(lin) || !finite3(ang)) {
-                fail(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(b));
+                fail(misc, 0u, MR_STEP_NONFINITE_RESULT);
+                failed = true;
             } else {
                 q = qscale(q, rsqrtf(qq));
             }
-            st3(s + kOffLin + b * 3, lin);
-            st3(s + kOffAng + b * 3, ang);
-            st3(s + kOffPos + b * 3, c);
-            st4(s + kOffQuat + b * 4, q);
+            st3(s + off_lin(nb) + b * 3, lin);
+            st3(s + off_ang(nb) + b * 3, ang);
+            st3(s + off_pos(nb) + b * 3, c);
+            st4(s + off_quat(nb) + b * 4, q);
         }
-        if (!ok(misc)) break;
+        if (__syncthreads_or(failed)) break;
     }
+    __syncthreads();
 
     // Commit: a failed control step publishes nothing (HBM keeps the
     // step-start state), except that a failed reset publishes the reset state.
-    const unsigned code = static_cast<unsigned>(ai(misc[kSmStatus]));
-    const bool success = code == MR_STEP_SUCCESS;
+    const unsigned failure = static_cast<unsigned>(ai(misc[kSmStatus]));
+    const bool success = failure == kNoFailure;
+    const unsigned code = success ? static_cast<unsigned>(MR_STEP_SUCCESS) : (failure & 0xffffu);
     float* qd = p.q + static_cast<size_t>(env) * nq;
     float* vd = p.v + static_cast<size_t>(env) * nv;
     float* obs = p.observations ? p.observations + static_cast<size_t>(item) * (nq + nv) : nullptr;
     if (success) {
-        for (int b = lane; b < nb; b += 32) {
-            st3(qd + b * 7, ld3(s + kOffPos + b * 3));
-            st4(qd + b * 7 + 3, ld4(s + kOffQuat + b * 4));
-            st3(vd + b * 6, ld3(s + kOffLin + b * 3));
-            st3(vd + b * 6 + 3, ld3(s + kOffAng + b * 3));
-            if (kComp) st3(p.q_comp + static_cast<size_t>(env) * nq + b * 7, ld3(s + kOffPosComp + b * 3));
+#pragma unroll 1
+        for (int i = tid; i < nq; i += nt) {
+            const int b = i / 7, k = i - 7 * b;
+            const float x = k < 3 ? s[off_pos(nb) + b * 3 + k] : s[off_quat(nb) + b * 4 + k - 3];
+            qd[i] = x;
+            if (obs) obs[i] = x;
         }
+#pragma unroll 1
+        for (int i = tid; i < nv; i += nt) {
+            const int b = i / 6, k = i - 6 * b;
+            const float x = k < 3 ? s[off_lin(nb) + b * 3 + k] : s[off_ang(nb) + b * 3 + k - 3];
+            vd[i] = x;
+            if (obs) obs[nq + i] = x;
+        }
+        if (kComp)
+#pragma unroll 1
+            for (int b = tid; b < nb; b += nt) st3(p.q_comp + static_cast<size_t>(env) * nq + b * 7, ld3(pos_comp + b * 3));
         if (cur_table != persistent)
-            for (int i = lane; i < mcount * kSceneSlotWords; i += 32) persistent[i] = cur_table[i];
-        if (lane == 0) {
+#pragma unroll 1
+            for (int i = tid; i < mcount * kSceneSlotWords; i += nt) persistent[i] = cur_table[i];
+        if (tid == 0) {
             p.manifold_count[env] = static_cast<std::uint32_t>(mcount);
             // A zero point count ends the table for host readers.
             if (mcount < kSceneManifolds) persistent[mcount * kSceneSlotWords + 7] = af(0);
         }
-    } else if (reset) {
-        for (int i = lane; i < nq; i += 32) qd[i] = srcq[i];
-        for (int i = lane; i < nv; i += 32) vd[i] = srcv[i];
-        if (kComp)
-            for (int b = lane; b < nb; b += 32) st3(p.q_comp + static_cast<size_t>(env) * nq + b * 7, f3(0.0f, 0.0f, 0.0f));
-        if (lane == 0) {
-            p.manifold_count[env] = 0u;
-            p.manifolds[static_cast<size_t>(env) * kTableWords + 7] = af(0);
+    } else {
+        // srcq / srcv are the reset state after a reset, else the resident one.
+#pragma unroll 1
+        for (int i = tid; i < nq; i += nt) {
+            const float x = srcq[i];
+            if (reset) qd[i] = x;
+            if (obs) obs[i] = x;
+        }
+#pragma unroll 1
+        for (int i = tid; i < nv; i += nt) {
+            const float x = srcv[i];
+            if (reset) vd[i] = x;
+            if (obs) obs[nq + i] = x;
+        }
+        if (reset) {
+            if (kComp)
+#pragma unroll 1
+                for (int b = tid; b < nb; b += nt) st3(p.q_comp + static_cast<size_t>(env) * nq + b * 7, f3(0.0f, 0.0f, 0.0f));
+            if (tid == 0) {
+                p.manifold_count[env] = 0u;
+                persistent[7] = af(0);
+            }
         }
     }
-    __syncwarp();
-    if (obs) {
-        for (int i = lane; i < nq; i += 32) obs[i] = qd[i];
-        for (int i = lane; i < nv; i += 32) obs[nq + i] = vd[i];
-    }
-    if (lane == 0) {
+    if (tid == 0) {
         const unsigned contacts = static_cast<unsigned>(ai(misc[kSmContacts]));
         if (p.status_codes) p.status_codes[item] = code;
         if (p.active_contacts) p.active_contacts[item] = success ? contacts : 0u;

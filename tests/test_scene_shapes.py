@@ -1,0 +1,70 @@
+"""The free-body kernel's launch shapes (warps per environment, shared memory)
+follow the body count and the environment count; no arithmetic does.  The
+first environments of a large world therefore end on the same bits as the
+same environments in a small one, on both sides of every rule, and also when
+a substep's contacts do not fit the small shape's shared memory."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import numi_lab_b200 as nb
+
+pytestmark = pytest.mark.gpu
+
+FEW = 6  # four warps per environment
+
+
+def _run(source, seed, envs, q, v, steps):
+    import torch
+
+    with nb.World(source, envs, substeps=4, velocity_iterations=8, control_dt=0.02, seed=seed) as w:
+        reps = -(-envs // FEW)
+        w.set_state(np.tile(q, (reps, 1))[:envs], np.tile(v, (reps, 1))[:envs])
+        _, status, _ = w.step(torch.zeros((steps, envs, 0), device="cuda"), wait=True)
+        assert int(status.abs().sum()) == 0
+        q1, v1, table = w.state()
+        return q1[:FEW], v1[:FEW], table[:FEW]
+
+
+def _same(a, b):
+    for name, x, y in zip(("q", "v", "manifolds"), a, b):
+        np.testing.assert_array_equal(x, y, err_msg=name)
+
+
+# One, two and four warps: small and large worlds below and above 592 and 1184
+# environments (four and eight per SM).
+@pytest.mark.parametrize("source,bodies,envs", [("pile", 9, 600), ("pile", 9, 1190), ("pile", 28, 1190), ("pile", 29, 600),
+                                                ("pile", 64, 1190), ("cylinder_pile", 23, 600), ("cylinder_pile", 23, 1190),
+                                                ("hull_pile", 29, 600)])
+def test_every_launch_shape_gives_the_same_bits(cuda_device, source, bodies, envs):
+    seed = nb.world.pile_seeds_by_body_count([bodies])[bodies]
+    q, v, _ = nb.sample_reset(source, seed, 7, 0, FEW)
+    few = _run(source, seed, FEW, q, v, 12)
+    many = _run(source, seed, envs, q, v, 12)
+    _same(few, many)
+
+
+def test_contacts_beyond_the_shared_arrays(cuda_device):
+    """28 upright bodies drawn together until they make about 160 contacts:
+    more than the 126 that the one-warp shape of a support-mapped world this
+    size keeps in shared memory (its 2800 words less the 1662 of the rest,
+    nine words per contact)."""
+
+    bodies, envs, shrink = 28, 1190, 0.25
+    seed = nb.world.pile_seeds_by_body_count([bodies])[bodies]
+    q, v, _ = nb.sample_reset("pile_gjk", seed, 7, 0, FEW)  # three layers
+    q = q.reshape(FEW, bodies, 7).copy()
+    q[:, :, :2] *= shrink
+    q[:, :, 2] = 0.05 + (q[:, :, 2] - q[:, :, 2].min()) * shrink
+    q[:, :, 3:] = (0.0, 0.0, 0.0, 1.0)
+    results = []
+    for n in (FEW, envs):
+        with nb.World("cylinder_pile", n, substeps=1, velocity_iterations=8, control_dt=0.005, seed=seed) as w:
+            reps = -(-n // FEW)
+            w.set_state(np.tile(q.reshape(FEW, -1), (reps, 1))[:n], np.tile(np.zeros_like(v), (reps, 1))[:n])
+            out = w.advance_host(np.zeros((1, n, 0), np.float32))
+            assert (out["status"] == 0).all() and out["contacts"].min() > 126
+            results.append(tuple(x[:FEW] for x in w.state()))
+    _same(*results)
