@@ -27,6 +27,13 @@
 // change x = H^-1 G^T lambda.  It is the reference's Jacobi block iteration
 // in generalized velocities (MetalWorldContact.metal:6655-7000), evaluated
 // without dense response columns.
+//
+// Instruction fetch bounds this kernel as much as issue does: 13 warps per SM
+// each sit at their own stage, so its whole code is the working set of the
+// instruction cache.  Loops whose body is more than a few instructions are
+// therefore rolled (`unroll 1`), or unrolled by two to four where their loads
+// are a chain.  4096 tree29 environments, four control steps: 270 KB of code
+// 6804 us, 207 KB 5598 us, the same bits.
 #pragma once
 
 #include "device_model.h"
@@ -124,6 +131,7 @@ __device__ void compute_drives(const Warp& w) {
     const float* v = w.s + w.L->v;
     const float* tgt = w.s + w.L->tgt;
     float* tau = w.s + w.L->tau;
+#pragma unroll 1
     for (int d = w.lane; d < M.nv; d += 32) {
         const unsigned flags = M.dof_flags[d];
         const float vel = v[d];
@@ -282,6 +290,7 @@ __device__ void kinematics(const Warp& w, const BodyConst& bc, BodyState<R>& st)
         Jd[3] = q[0]; Jd[4] = q[1]; Jd[5] = q[2];
         Jd[6] = b < 3 ? 1.0f : 0.0f;
     }
+#pragma unroll 1
     for (int l = 1; l <= T.n_levels; ++l) {
         const float3 cp = shfl3(st.c, par);
         const float4 qp = shfl4(st.qr, par);
@@ -419,8 +428,10 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
     const int first_child = mine ? T.child_offsets[b] : 0;
     const int n_children = mine ? T.child_offsets[b + 1] - first_child : 0;
     float3 acc_ang = f3(0.0f, 0.0f, 0.0f), acc_lin = f3(0.0f, 0.0f, 0.0f);
+#pragma unroll 1
     for (int l = T.n_levels; l >= 0; --l) {
         const bool active = my_depth == l;
+#pragma unroll 1
         for (int k = 0; k < T.level_children[l]; ++k) {
             const bool take = active && k < n_children;
             const int src = take ? T.children[first_child + k] : b;
@@ -546,6 +557,7 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
         const R inv = R(1) / lkk;
         rowk[k] = static_cast<float>(lkk);
         const int na = T.dof_depth[k];
+#pragma unroll 2
         for (int t = 0; t < na; ++t) {
             const int j = T.anc[b][t];
             const float* jd = J + j * kJStride;
@@ -563,6 +575,7 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
 
     // Forward acceleration sweep: the parent's acceleration by shuffle.
     const int par = (mine && b > 0) ? T.parent[b] : b;
+#pragma unroll 1
     for (int l = 1; l <= T.n_levels; ++l) {
         const float3 pa = shfl3(acc_ang, par);
         const float3 plin = shfl3(acc_lin, par);
@@ -584,6 +597,7 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
     __syncwarp();
     // v_free = v + h qdd.
     float* vf = s + L.vf;
+#pragma unroll 1
     for (int d = b; d < M.nv; d += 32) {
         const float a = qdd[d];
         const float nvv = v[d] + M.h * a;
@@ -606,6 +620,7 @@ __device__ bool integrate_free(const Warp& w) {
     float* v = s + L.v;
     float* qc = s + L.qcomp;
     const float* vf = s + L.vf;
+#pragma unroll 1
     for (int d = w.lane; d < M.nv; d += 32) {
         v[d] = vf[d];
         const int qi = M.dof_q[d];
@@ -802,12 +817,14 @@ __device__ int pair_manifold(const DeviceModel& M, const float* pose, const floa
         const float sep = dot3(plane.normal, surface - plane.center);
         if (sep <= accepted) append(surface, sep, feature_key(MR_SHAPE_SPHERE, 0u));
     } else if (cls == MR_COLLISION_PAIR_CAPSULE_PLANE) {
+#pragma unroll 1
         for (int e = 0; e < 2; ++e) {
             const float3 surface = (e == 0 ? fin.ep0 : fin.ep1) - plane.normal * fin.radius;
             const float sep = dot3(plane.normal, surface - plane.center);
             if (sep <= accepted) append(surface, sep, feature_key(MR_SHAPE_CAPSULE, static_cast<unsigned>(e)));
         }
     } else if (cls == MR_COLLISION_PAIR_BOX_PLANE) {
+#pragma unroll 1
         for (unsigned vtx = 0; vtx < 8u; ++vtx) {
             const float3 local = f3((vtx & 1u) ? fin.half.x : -fin.half.x, (vtx & 2u) ? fin.half.y : -fin.half.y,
                                     (vtx & 4u) ? fin.half.z : -fin.half.z);
@@ -843,6 +860,7 @@ __device__ int pair_manifold(const DeviceModel& M, const float* pose, const floa
             const float3 ot = qrot(rotA, ld3(slot + 4));
             transported = ot - nw * dot3(ot, nw);
             old_age = slot[3];
+#pragma unroll 1
             for (int i = 0; i < old_count; ++i) {
                 const float* op = slot + 8 + i * 12;
                 const float3 pa = posA + qrot(rotA, ld3(op));
@@ -868,16 +886,19 @@ __device__ int pair_manifold(const DeviceModel& M, const float* pose, const floa
     // Raw contacts refresh a candidate with the same features, else one
     // within the merge distance, else join as new points.
     const float merge2 = thr.z * thr.z;
+#pragma unroll 1
     for (int r = 0; r < nraw; ++r) {
         const float* rr = raw + r * kCandidateWords;
         const float3 la = ld3(rr + kCdLa), lb = ld3(rr + kCdLb);
         const int fa = as_int(rr[kCdFa]), fb = as_int(rr[kCdFb]);
         int match = -1;
+#pragma unroll 1
         for (int k = 0; k < nc; ++k) {
             const float* g = scratch + (ids[k] & 15u) * kCandidateWords;
             if (as_int(g[kCdFa]) == fa && as_int(g[kCdFb]) == fb) { match = k; break; }
         }
         if (match < 0) {
+#pragma unroll 1
             for (int k = 0; k < nc; ++k) {
                 const float* g = scratch + (ids[k] & 15u) * kCandidateWords;
                 const float3 da = ld3(g + kCdLa) - la;
@@ -896,6 +917,7 @@ __device__ int pair_manifold(const DeviceModel& M, const float* pose, const floa
     // cannot change the result (the final order is canonical by feature), so
     // the separation sort and the reduction run only for larger sets.
     if (nc > kManifoldPoints) {
+#pragma unroll 1
         for (int i = 1; i < nc; ++i) {
             const unsigned char val = ids[i];
             const float* gv = scratch + (val & 15u) * kCandidateWords;
@@ -923,10 +945,12 @@ __device__ int pair_manifold(const DeviceModel& M, const float* pose, const floa
         int chosen_count = 1;
         const float3 w0 = ld3(scratch + (ids[0] & 15u) * kCandidateWords + kCdWp);
         float3 w1 = w0;
+#pragma unroll 1
         for (int stage = 1; stage < kManifoldPoints; ++stage) {
             int best = -1;
             float best_score = -1.0f;
             unsigned long long best_feature = ~0ull;
+#pragma unroll 1
             for (int i = 0; i < nc; ++i) {
                 if (selected & (1u << i)) continue;
                 const float* gi = scratch + (ids[i] & 15u) * kCandidateWords;
@@ -940,6 +964,7 @@ __device__ int pair_manifold(const DeviceModel& M, const float* pose, const floa
                     score = fabsf(dot3(cross3(w1 - w0, wi - w0), nw));
                 } else {
                     score = INFINITY;
+#pragma unroll 1
                     for (int k = 0; k < chosen_count; ++k) {
                         const int ck = static_cast<int>((chosen >> (8 * k)) & 0xffu);
                         const float3 dl = wi - ld3(scratch + (ids[ck] & 15u) * kCandidateWords + kCdWp);
@@ -963,11 +988,14 @@ __device__ int pair_manifold(const DeviceModel& M, const float* pose, const floa
             }
         }
         unsigned packed = 0u;
+#pragma unroll 1
         for (int k = 0; k < chosen_count; ++k) packed |= static_cast<unsigned>(ids[(chosen >> (8 * k)) & 0xffu]) << (8 * k);
+#pragma unroll 1
         for (int k = 0; k < chosen_count; ++k) ids[k] = static_cast<unsigned char>((packed >> (8 * k)) & 0xffu);
         nc = chosen_count;
     }
     // Canonical order by feature pair.
+#pragma unroll 1
     for (int i = 1; i < nc; ++i) {
         const unsigned char val = ids[i];
         const unsigned long long f = record_key(scratch + (val & 15u) * kCandidateWords);
@@ -985,6 +1013,7 @@ __device__ int pair_manifold(const DeviceModel& M, const float* pose, const floa
     slot[3] = old_ok ? fminf(old_age + 1.0f, 65535.0f) : 0.0f;
     st3(slot + 4, qrotinv(rotA, tw));
     slot[7] = as_float(nc);
+#pragma unroll 1
     for (int i = 0; i < kManifoldPoints; ++i) {
         float* op = slot + 8 + i * 12;
         if (i < nc) {
@@ -1160,6 +1189,7 @@ __device__ void group_manifold(const DeviceModel& M, const float* pose, const fl
     unsigned my_id = 0xffu;
     {
         unsigned m = kept_mask;
+#pragma unroll 1
         for (int k = 0; k < sl && m != 0u; ++k) m &= m - 1u;
         if (sl < nc) {
             const unsigned i = static_cast<unsigned>(__ffs(m) - 1);
@@ -1169,6 +1199,7 @@ __device__ void group_manifold(const DeviceModel& M, const float* pose, const fl
     // Raw contacts in feature order refresh the first candidate with the
     // same features, else the first within the merge distance, else join.
     const float merge2 = thr.z * thr.z;
+#pragma unroll 1
     for (unsigned m = raw_mask; m != 0u; m &= m - 1u) {
         const int r = __ffs(m) - 1;
         const float* rr = raw + r * kCandidateWords;
@@ -1210,7 +1241,7 @@ __device__ void group_manifold(const DeviceModel& M, const float* pose, const fl
         // reduceCandidates: order by (separation, features), then greedy
         // selection with the precision-independent tie rule of pair_manifold.
         int rank = 0;
-#pragma unroll
+#pragma unroll 1
         for (int j = 0; j < kMaxCandidates; ++j) {
             const float sj = __shfl_sync(gmask, my_sep, j, 16);
             const unsigned fj = __shfl_sync(gmask, my_fa, j, 16);
@@ -1221,7 +1252,7 @@ __device__ void group_manifold(const DeviceModel& M, const float* pose, const fl
             }
         }
         unsigned long long order = 0ull;  // candidate lane of each rank
-#pragma unroll
+#pragma unroll 1
         for (int i = 0; i < kMaxCandidates; ++i) {
             const unsigned who = group_ballot(gmask, gbase, sl < nc && rank == i);
             if (i < nc) order |= static_cast<unsigned long long>(__ffs(who) - 1) << (4 * i);
@@ -1232,6 +1263,7 @@ __device__ void group_manifold(const DeviceModel& M, const float* pose, const fl
         int chosen_count = 1;
         const float3 w0 = shfl3g(my_wp, c0, gmask);
         float3 w1 = w0, w2 = w0;
+#pragma unroll 1
         for (int stage = 1; stage < kManifoldPoints; ++stage) {
             float score;
             if (stage == 1) {
@@ -1253,7 +1285,7 @@ __device__ void group_manifold(const DeviceModel& M, const float* pose, const fl
             int best = -1;
             float best_score = -1.0f;
             unsigned long long best_feature = ~0ull;
-#pragma unroll
+#pragma unroll 1
             for (int i = 0; i < kMaxCandidates; ++i) {
                 const int k = static_cast<int>((order >> (4 * i)) & 0xfull);
                 const float sc = __shfl_sync(gmask, score, k, 16);
@@ -1489,6 +1521,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
         const int g = lane >> 4, sl = lane & 15, gbase = lane & 16;
         const unsigned gmask = g ? 0xffff0000u : 0x0000ffffu;
         const int nheavy = __popc(heavy_mask);
+#pragma unroll 1
         for (int first = 0; first < nheavy; first += 2) {
             unsigned m = heavy_mask;
             for (int k = 0; k < first + g && m != 0u; ++k) m &= m - 1u;
@@ -1575,6 +1608,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
         const float compliance = ra.z + rb.z;
         const float dissipation = ra.w + rb.w;
         const float rest = M.shape_offsets[sa].y + M.shape_offsets[sb].y;
+#pragma unroll 1
         for (int i = 0; i < npoints; ++i) {
             const float* op = slot + 8 + i * 12;
             float* c = C + (base + i) * kContactWords;
@@ -1623,6 +1657,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
         const int na = T.anc_count[b];
         float* g = Y + lane * 3 * ma;
         float rel[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll 2
         for (int k = 0; k < na; ++k) {
             const int d = T.anc[b][k];
             // Point-Jacobian column: a x (x - o) for rotations, a for translations.
@@ -1667,6 +1702,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
         if (lane == 0) misc[kMiscIslands] = as_float(max(as_int(misc[kMiscIslands]), 1));
         // Y = L^-T G^T per contact row, in place over the ancestor positions.
         const int nrows = 3 * total;
+#pragma unroll 1
         for (int row = lane; row < nrows; row += 32) {
             const int c = row / 3, r = row - 3 * (row / 3);
             const int b = as_int(C[c * kContactWords + kCwBody]);
@@ -1697,11 +1733,13 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
                 for (int t = 0; t < kRegisterChain; ++t)
                     if (t < na) y[t] = yr[t];
             } else {
+#pragma unroll 1
                 for (int t = na - 1; t >= 0; --t) {
                     const int k = T.anc[b][t];
                     const float* rowk = Lm + k * (k + 1) / 2;
                     const float yt = y[t] / rowk[k];
                     y[t] = yt;
+#pragma unroll 1
                     for (int u = 0; u < t; ++u) y[u] -= rowk[T.anc[b][u]] * yt;
                 }
             }
@@ -1723,6 +1761,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
             if (d < nv) {
                 z[d] = 0.0f;
                 int cnt = 0;
+#pragma unroll 2
                 for (int j = 0; j < total; ++j) {
                     const int t = T.pos[as_int(C[j * kContactWords + kCwBody])][d];
                     if (t != kNone) dlist[d * ncap + cnt++] = static_cast<std::uint16_t>((t << 5) | j);
@@ -1738,20 +1777,28 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
             const int b = as_int(c[kCwBody]);
             const int na = T.anc_count[b];
             const float* yc = Y + lane * 3 * ma;
-            float Wm[3][3];
-            for (int r = 0; r < 3; ++r)
-                for (int cc = 0; cc <= r; ++cc) {
-                    float acc = 0.0f;
-                    for (int t = 0; t < na; ++t) acc = fmaf(yc[r * ma + t], yc[cc * ma + t], acc);
-                    Wm[r][cc] = acc;
-                    Wm[cc][r] = acc;
-                }
+            float Wm[3][3] = {};
+#pragma unroll 2
+            for (int t = 0; t < na; ++t) {
+                const float y0 = yc[t], y1 = yc[ma + t], y2 = yc[2 * ma + t];
+                Wm[0][0] = fmaf(y0, y0, Wm[0][0]);
+                Wm[1][0] = fmaf(y1, y0, Wm[1][0]);
+                Wm[1][1] = fmaf(y1, y1, Wm[1][1]);
+                Wm[2][0] = fmaf(y2, y0, Wm[2][0]);
+                Wm[2][1] = fmaf(y2, y1, Wm[2][1]);
+                Wm[2][2] = fmaf(y2, y2, Wm[2][2]);
+            }
+            Wm[0][1] = Wm[1][0];
+            Wm[0][2] = Wm[2][0];
+            Wm[1][2] = Wm[2][1];
             float rowsum = 0.0f;
+#pragma unroll 1
             for (int j = 0; j < total; ++j) {
                 const int bj = as_int(C[j * kContactWords + kCwBody]);
                 const int n = T.lcp[b][bj];
                 const float* yj = Y + j * 3 * ma;
                 float acc = 0.0f;
+#pragma unroll 4
                 for (int t = 0; t < n; ++t) acc = fmaf(yc[t], yj[t], acc);
                 rowsum += fabsf(acc);
             }
@@ -1774,6 +1821,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
         // lane per DoF accumulates z += Y delta.  Sweep -1 applies the warm start.
         const int iters = velocity_iterations + (final_substep ? final_iterations : 0);
         float zcomp[2] = {0.0f, 0.0f};  // kComp: compensation of the z sums
+#pragma unroll 1
         for (int it = -1; it < iters; ++it) {
             if (it >= 0 && lane < total) {
                 float* c = C + lane * kContactWords;
@@ -1781,6 +1829,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
                 const int na = T.anc_count[b];
                 const float* yc = Y + lane * 3 * ma;
                 float u0 = c[kCwUfree + 0], u1 = c[kCwUfree + 1], u2 = c[kCwUfree + 2];
+#pragma unroll 4
                 for (int t = 0; t < na; ++t) {
                     const float zk = z[T.anc[b][t]];
                     u0 = fmaf(yc[t], zk, u0);
@@ -1854,7 +1903,9 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
                 dv = f3(xr[0], xr[1], xr[2]);
                 dw = f3(xr[3], xr[4], xr[5]);
             }
-            for (int l = 1; l <= T.n_levels; ++l) {
+#pragma unroll 1
+        #pragma unroll 1
+    for (int l = 1; l <= T.n_levels; ++l) {
                 const float3 pw = shfl3(dw, par);
                 const float3 pv = shfl3(dv, par);
                 if (my_depth == l) {
@@ -1887,6 +1938,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
     __syncwarp();
 
     // Joint limits on the post-solve velocity (mr_world_project_joint_limits).
+#pragma unroll 1
     for (int d = lane; d < nv; d += 32) {
         const unsigned flags = M.dof_flags[d];
         float vel = v[d];
@@ -1903,6 +1955,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
     // Integration from the substep-start configuration
     // (mr_world_integrate_contact_state; no angle reduction).
     float* qc = s + L.qcomp;
+#pragma unroll 1
     for (int d = lane; d < nv; d += 32) {
         const int qi = M.dof_q[d];
         if (qi >= 0 && !(M.floating && d < 6)) q[qi] = kComp ? kahan_madd(q[qi], h, v[d], qc[qi]) : q[qi] + h * v[d];
@@ -1974,11 +2027,13 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
     const bool reset = p.reset_masks != nullptr && p.reset_masks[item] != 0u;
     const float* srcq = (reset ? p.reset_q : p.q) + static_cast<size_t>(env) * nq;
     const float* srcv = (reset ? p.reset_v : p.v) + static_cast<size_t>(env) * nv;
+#pragma unroll 1
     for (int i = lane; i < nq; i += 32) {
         const float x = srcq[i];
         s[layout.q + i] = x;
         s[layout.qc + i] = x;
     }
+#pragma unroll 1
     for (int i = lane; i < nv; i += 32) {
         const float x = srcv[i];
         s[layout.v + i] = x;
@@ -1991,6 +2046,7 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
     }
     misc[lane] = 0.0f;
     __syncwarp();
+#pragma unroll 1
     for (int a = lane; a < M.action_count; a += 32)
         s[layout.tgt + M.action_dof[a]] =
             p.action_rows != nullptr ? p.action_rows[item][a] : p.actions[static_cast<size_t>(item) * M.action_count + a];
@@ -2000,6 +2056,7 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
         float* slots = s + layout.manifolds;
         const int words = M.np * kManifoldWords;
         const float* src = p.manifolds + static_cast<size_t>(env) * words;
+#pragma unroll 4
         for (int i = lane; i < words; i += 32) {
             const int pair = i / kManifoldWords;
             slots[pair * kSlotStride + (i - pair * kManifoldWords)] = reset ? 0.0f : src[i];
@@ -2011,6 +2068,7 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
     BodyState<R> st;
     __syncwarp();
 
+#pragma unroll 1
     for (int sub = 0; sub < p.substeps; ++sub) {
         compute_drives(w);
         __syncwarp();
@@ -2032,11 +2090,13 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
     const float* qsrc = s + (success ? layout.q : layout.qc);
     const float* vsrc = s + (success ? layout.v : layout.vc);
     float* obs = p.observations ? p.observations + static_cast<size_t>(item) * (nq + nv) : nullptr;
+#pragma unroll 1
     for (int i = lane; i < nq; i += 32) {
         const float x = qsrc[i];
         qd[i] = x;
         if (obs) obs[i] = x;
     }
+#pragma unroll 1
     for (int i = lane; i < nv; i += 32) {
         const float x = vsrc[i];
         vd[i] = x;
@@ -2051,6 +2111,7 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
         const int words = M.np * kManifoldWords;
         float* dst = p.manifolds + static_cast<size_t>(env) * words;
         const float* slots = s + layout.manifolds;
+#pragma unroll 4
         for (int i = lane; i < words; i += 32) {
             const int pair = i / kManifoldWords;
             dst[i] = success ? slots[pair * kSlotStride + (i - pair * kManifoldWords)] : 0.0f;
