@@ -57,6 +57,16 @@ __device__ __forceinline__ bool qnormalize(float4 in, float4& out, bool require_
     return finite4(out);
 }
 
+// Normalises a product of unit quaternions.  Near one, 1 / |q| is its Taylor
+// polynomial in |q|^2 - 1 (the next term, 5/16 (1e-3)^3, is below FP32
+// rounding): no square root or division on the way down a kinematic chain.
+__device__ __forceinline__ bool qrenormalize(float4 in, float4& out) {
+    const float d = qdot(in, in) - 1.0f;
+    if (!(fabsf(d) <= 1.0e-3f)) return qnormalize(in, out, false);
+    out = qscale(in, fmaf(d, fmaf(d, 0.375f, -0.5f), 1.0f));
+    return true;
+}
+
 // Exponential-map increment for a world angular displacement h*omega,
 // composed on the left: q' = normalize(exp(h w) * q).
 __device__ __forceinline__ float4 so3_increment(float3 rv, bool reduce_angle) {

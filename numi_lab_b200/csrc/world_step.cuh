@@ -229,11 +229,16 @@ __device__ __forceinline__ void body_inertia(const DeviceModel& M, int b, float4
 }
 
 // ---------------------------------------------------------------------------
-// Forward kinematics (ArticulatedABA.metal:735-905): lane b computes body b
-// at its tree level from its parent's pose and twist, read from the parent
-// lane's registers by warp shuffle.  Leaves the pose in shared memory (for
-// collision) and the joint axis / origin of the body's DoF in the Jacobian
-// table; bias accelerations, offset and subspace stay in registers.
+// Forward kinematics (ArticulatedABA.metal:735-905): lane b owns body b.
+// Only what a body needs from its parent goes level by level, by warp
+// shuffle from the parent's lane: the orientation (one quaternion product
+// with the joint's own transform), then position and twist (a rotated offset
+// and one cross product).  The joint transforms, the rotated anchors and
+// axes, and the bias accelerations are computed by all lanes at once around
+// those two sweeps, because a level keeps at most a few lanes busy.  Leaves
+// the pose in shared memory (for collision) and the joint axis / origin of
+// the body's DoF in the Jacobian table; bias accelerations, offset and
+// subspace stay in registers.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float3 shfl3(float3 a, int src) {
     return f3(__shfl_sync(0xffffffffu, a.x, src), __shfl_sync(0xffffffffu, a.y, src), __shfl_sync(0xffffffffu, a.z, src));
@@ -290,63 +295,79 @@ __device__ void kinematics(const Warp& w, const BodyConst& bc, BodyState<R>& st)
         Jd[3] = q[0]; Jd[4] = q[1]; Jd[5] = q[2];
         Jd[6] = b < 3 ? 1.0f : 0.0f;
     }
+    const bool child = my_depth >= 1;
+    const bool has = child && bc.dof >= 0;
+    const bool prismatic = child && bc.type == MR_JOINT_PRISMATIC;
+    const bool turns = has && !prismatic;
+    const float3 zero = f3(0.0f, 0.0f, 0.0f);
+    // Joint transform in the parent's frame.
+    float4 local = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+    float3 axis = zero, anchor = zero;
+    float qdj = 0.0f;
+    if (child) {
+        const float4 pr = M.parent_rotation[b];
+        const float3 unit = xyz(M.axis[b]);
+        axis = qrot(pr, unit);
+        anchor = xyz(M.parent_anchor[b]);
+        local = pr;
+        if (has) {
+            const float qj = q[bc.qidx];
+            qdj = v[bc.dof];
+            if (turns) {
+                float sh, ch;
+                sincosf(0.5f * qj, &sh, &ch);
+                local = qmul(pr, make_float4(unit.x * sh, unit.y * sh, unit.z * sh, ch));
+            } else {
+                anchor = anchor + axis * qj;
+            }
+        }
+        local = qmul(local, M.child_rotation_conj[b]);
+    }
+#pragma unroll 1
+    for (int l = 1; l <= T.n_levels; ++l) {
+        const float4 qp = shfl4(st.qr, par);
+        if (my_depth == l && !qrenormalize(qmul(qp, local), st.qr)) {
+            set_status(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(b));
+            st.qr = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+        }
+    }
+    const float4 qp = shfl4(st.qr, par);
+    const float3 ja = qrot(qp, axis);
+    const float3 ptj = qrot(qp, anchor);  // parent COM -> joint
+    const float3 ca = child ? qrot(st.qr, xyz(M.child_anchor[b])) : zero;
+    const float3 rate = ja * qdj;
+    const float3 dw = turns ? rate : zero;
+    const float3 dv = prismatic ? rate : -cross3(dw, ca);
+    if (child) st.r = ptj - ca;
 #pragma unroll 1
     for (int l = 1; l <= T.n_levels; ++l) {
         const float3 cp = shfl3(st.c, par);
-        const float4 qp = shfl4(st.qr, par);
         const float3 wp = shfl3(st.w, par);
         const float3 vp = shfl3(st.v, par);
         if (my_depth == l) {
-            const float3 axis = xyz(M.axis[b]);
-            const float4 pj = qmul(qp, M.parent_rotation[b]);
-            float4 motion = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-            float qj = 0.0f, qdj = 0.0f;
-            const bool has = bc.dof >= 0;
-            const bool prismatic = bc.type == MR_JOINT_PRISMATIC;
-            if (has) {
-                qj = q[bc.qidx];
-                qdj = v[bc.dof];
-                if (!prismatic) {
-                    float sh, ch;
-                    sincosf(0.5f * qj, &sh, &ch);
-                    motion = make_float4(axis.x * sh, axis.y * sh, axis.z * sh, ch);
-                }
-            }
-            float4 qb;
-            if (!qnormalize(qmul(qmul(pj, motion), M.child_rotation_conj[b]), qb, false)) {
-                set_status(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(b));
-                qb = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-            }
-            const float3 ja = qrot(pj, axis);
-            float3 jp = cp + qrot(qp, xyz(M.parent_anchor[b]));
-            if (prismatic) jp = jp + ja * qj;
-            const float3 ca = qrot(qb, xyz(M.child_anchor[b]));
-            const float3 cb = jp - ca;
-            const float3 ptj = jp - cp;
-            const float3 zero = f3(0.0f, 0.0f, 0.0f);
-            const float3 wb = wp + ((has && !prismatic) ? ja * qdj : zero);
-            const float3 vb = vp + cross3(wp, ptj) + (prismatic ? ja * qdj : zero) - cross3(wb, ca);
-            const float3 ma = (has && !prismatic) ? ja : zero;
-            const float3 ml = prismatic ? ja : (has ? -cross3(ja, ca) : zero);
-            st.ba = (has && !prismatic) ? cross3(wp, ja) * qdj : zero;
-            const float3 pc = prismatic ? cross3(wp, ja) * (2.0f * qdj) : zero;
-            st.bl = cross3(wp, cross3(wp, ptj)) + pc - cross3(st.ba, ca) - cross3(wb, cross3(wb, ca));
-            st.c = cb;
-            st.qr = qb;
-            st.w = wb;
-            st.v = vb;
-            st.r = cb - cp;
-            st.s[0] = ma.x; st.s[1] = ma.y; st.s[2] = ma.z;
-            st.s[3] = ml.x; st.s[4] = ml.y; st.s[5] = ml.z;
-            if (has) {
-                float* Jd = J + bc.dof * kJStride;
-                Jd[0] = ja.x; Jd[1] = ja.y; Jd[2] = ja.z;
-                Jd[3] = jp.x; Jd[4] = jp.y; Jd[5] = jp.z;
-                Jd[6] = prismatic ? 1.0f : 0.0f;
-            }
-            if (!finite3(cb) || !finite3(wb) || !finite3(vb) || !finite3(st.bl))
-                set_status(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(b));
+            st.c = cp + st.r;
+            st.w = wp + dw;
+            st.v = vp + cross3(wp, st.r) + dv;
         }
+    }
+    const float3 cp = shfl3(st.c, par);
+    const float3 wp = shfl3(st.w, par);
+    if (child) {
+        const float3 jp = cp + ptj;
+        const float3 ml = prismatic ? ja : (has ? -cross3(ja, ca) : zero);
+        if (turns) st.ba = cross3(wp, rate);
+        const float3 pc = prismatic ? 2.0f * cross3(wp, rate) : zero;
+        st.bl = cross3(wp, cross3(wp, ptj)) + pc - cross3(st.ba, ca) - cross3(st.w, cross3(st.w, ca));
+        if (turns) { st.s[0] = ja.x; st.s[1] = ja.y; st.s[2] = ja.z; }
+        st.s[3] = ml.x; st.s[4] = ml.y; st.s[5] = ml.z;
+        if (has) {
+            float* Jd = J + bc.dof * kJStride;
+            Jd[0] = ja.x; Jd[1] = ja.y; Jd[2] = ja.z;
+            Jd[3] = jp.x; Jd[4] = jp.y; Jd[5] = jp.z;
+            Jd[6] = prismatic ? 1.0f : 0.0f;
+        }
+        if (!finite3(st.c) || !finite3(st.w) || !finite3(st.v) || !finite3(st.bl))
+            set_status(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(b));
     }
     if (mine) {
         float* pb = pose + b * kPoseStride;
