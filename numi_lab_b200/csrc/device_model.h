@@ -41,6 +41,10 @@ struct alignas(16) DeviceTables {
     std::uint8_t lcp[kMaxBodies][kMaxBodies];// common prefix length of anc[a], anc[b]
     std::uint8_t level_children[kMaxBodies]; // most children of a body at each depth
     std::uint8_t pad[7];
+    // Factor rows hold only their ancestors: row k starts here, its entry t
+    // belongs to the t-th ancestor DoF and its last entry is the diagonal.
+    std::uint16_t row_start[kMaxDofs];
+    std::uint16_t factor_words, reserved1[7];
 };
 
 struct alignas(16) DeviceModel {

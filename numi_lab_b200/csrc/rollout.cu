@@ -229,6 +229,12 @@ numi::DeviceModel numi::rt::pack_model(const numi::CompiledModel& m, float h) {
             }
         }
         t.child_offsets[nb] = static_cast<std::uint8_t>(d.child_offsets[nb]);
+        std::uint16_t row = 0;
+        for (std::uint32_t dof = 0; dof < w.nv; ++dof) {
+            t.row_start[dof] = row;
+            row = static_cast<std::uint16_t>(row + d.dof_anc_count[dof] + 1);
+        }
+        t.factor_words = row;
         std::memset(t.level_children, 0, sizeof(t.level_children));
         for (int b = 0; b < nb; ++b) {
             const int children = d.child_offsets[b + 1] - d.child_offsets[b];
@@ -272,7 +278,7 @@ void numi::rt::make_plan(const numi::CompiledModel& m, float h, KernelPlan& plan
             (compensated ? plan.layout_comp : plan.layout)[quality] =
                 numi::make_layout(static_cast<int>(m.articulated_body_count), nv, static_cast<int>(m.world.nq),
                                   static_cast<int>(m.world.pair_count), ncap, static_cast<int>(m.max_ancestor_dofs), narrow_words,
-                                  plan.contact, compensated, quality ? numi::quality_workspace_doubles(nv, ncap) : 0);
+                                  plan.dmodel.tables.factor_words, plan.contact, compensated, quality ? numi::quality_workspace_doubles(nv, ncap) : 0);
     int device = 0;
     check(cudaGetDevice(&device), "cudaGetDevice");
     cudaDeviceProp prop{};

@@ -388,7 +388,9 @@ __device__ void kinematics(const Warp& w, const BodyConst& bc, BodyState<R>& st)
 // from the root's 6x6 factorisation): eliminating a DoF's descendants
 // leaves its body's articulated inertia, so L_kk = sqrt(D_k) and
 // L_kj = U_k . S_j(c_b) / L_kk for the ancestor DoFs j, with S_j moved to
-// body b's COM.
+// body b's COM.  Rows hold their ancestors only: an ancestor's position in a
+// contact body's list is its position in the rows of the DoFs below it, so
+// the substitution reads a row by consecutive words.
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float* factor) {
@@ -573,11 +575,11 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
     // Joint rows of the factor.
     if (factor != nullptr && mine && b > 0 && bc.dof >= 0) {
         const int k = bc.dof;
-        float* rowk = factor + k * (k + 1) / 2;
+        float* rowk = factor + T.row_start[k];
         const R lkk = sqrt(st.D);
         const R inv = R(1) / lkk;
-        rowk[k] = static_cast<float>(lkk);
         const int na = T.dof_depth[k];
+        rowk[na] = static_cast<float>(lkk);
 #pragma unroll 2
         for (int t = 0; t < na; ++t) {
             const int j = T.anc[b][t];
@@ -590,7 +592,7 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
                 const float3 lin = cross3(ax, st.c - f3(jd[3], jd[4], jd[5]));
                 val = st.U[0] * ax.x + st.U[1] * ax.y + st.U[2] * ax.z + st.U[3] * lin.x + st.U[4] * lin.y + st.U[5] * lin.z;
             }
-            rowk[j] = static_cast<float>(val * inv);
+            rowk[t] = static_cast<float>(val * inv);
         }
     }
 
@@ -1660,7 +1662,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
             c[kCwMuU] = mu_s;
             c[kCwMuV] = mu_d;
             c[kCwRelax] = restitution;
-            c[kCwDelta + 0] = rthreshold;
+            c[kCwUfree + 0] = rthreshold;
         }
     }
     __syncwarp();
@@ -1693,6 +1695,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
                 rel[r] = fmaf(gv, vk, rel[r]);
             }
         }
+        const float rthreshold = c[kCwUfree + 0];
         for (int r = 0; r < 3; ++r) c[kCwUfree + r] = rel[r];
         // Normal row: critically damped stabilisation clamped to the maximum
         // depenetration speed, plus restitution on a new impact.
@@ -1704,7 +1707,6 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
         float stab = -h * err / (tau_c * tau_c * den);
         stab = fminf(fmaxf(stab, 0.0f), M.max_depenetration);
         const float restitution = c[kCwRelax];
-        const float rthreshold = c[kCwDelta + 0];
         if (flags & 1) {
             const float incoming = rel[0] - c[kCwTarget + 0];
             if (incoming < -rthreshold) stab = fmaxf(stab, -restitution * incoming);
@@ -1737,17 +1739,17 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
 #pragma unroll
                 for (int t = 0; t < kRegisterChain; ++t) {
                     const int k = t < na ? T.anc[b][t] : 0;
-                    off[t] = k * (k + 1) / 2;
+                    off[t] = T.row_start[k];
                     yr[t] = t < na ? y[t] : 0.0f;
                 }
 #pragma unroll
                 for (int t = kRegisterChain - 1; t >= 0; --t) {
                     if (t < na) {
                         const float* rowk = Lm + off[t];
-                        const float yt = yr[t] / rowk[T.anc[b][t]];
+                        const float yt = yr[t] / rowk[t];
                         yr[t] = yt;
 #pragma unroll
-                        for (int u = 0; u < t; ++u) yr[u] -= rowk[T.anc[b][u]] * yt;
+                        for (int u = 0; u < t; ++u) yr[u] -= rowk[u] * yt;
                     }
                 }
 #pragma unroll
@@ -1756,12 +1758,11 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
             } else {
 #pragma unroll 1
                 for (int t = na - 1; t >= 0; --t) {
-                    const int k = T.anc[b][t];
-                    const float* rowk = Lm + k * (k + 1) / 2;
-                    const float yt = y[t] / rowk[k];
+                    const float* rowk = Lm + T.row_start[T.anc[b][t]];
+                    const float yt = y[t] / rowk[t];
                     y[t] = yt;
 #pragma unroll 1
-                    for (int u = 0; u < t; ++u) y[u] -= rowk[T.anc[b][u]] * yt;
+                    for (int u = 0; u < t; ++u) y[u] -= rowk[u] * yt;
                 }
             }
         }
@@ -1910,6 +1911,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
             const int my_depth = mine ? T.depth[lane] : -1;
             const int par = (mine && lane > 0) ? T.parent[lane] : lane;
             float3 dw = f3(0.0f, 0.0f, 0.0f), dv = f3(0.0f, 0.0f, 0.0f);
+            const float lkk = mine && lane > 0 && bc.dof >= 0 ? static_cast<float>(sqrt(st.D)) : 1.0f;  // as written by the ABA
             if (lane == 0 && T.floating) {
                 float xr[6];
 #pragma unroll
@@ -1934,7 +1936,6 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
                     dv = pv + cross3(pw, st.r);
                     if (bc.dof >= 0) {
                         const int k = bc.dof;
-                        const float lkk = static_cast<float>(sqrt(st.D));  // = L_kk as written by the ABA
                         const float sum = static_cast<float>(st.U[0] * dw.x + st.U[1] * dw.y + st.U[2] * dw.z +
                                                              st.U[3] * dv.x + st.U[4] * dv.y + st.U[5] * dv.z);
                         const float xk = (z[k] - sum / lkk) / lkk;
@@ -2052,13 +2053,11 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
     for (int i = lane; i < nq; i += 32) {
         const float x = srcq[i];
         s[layout.q + i] = x;
-        s[layout.qc + i] = x;
     }
 #pragma unroll 1
     for (int i = lane; i < nv; i += 32) {
         const float x = srcv[i];
         s[layout.v + i] = x;
-        s[layout.vc + i] = x;
         s[layout.tgt + i] = 0.0f;
     }
     if (kComp) {
@@ -2105,11 +2104,12 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
     }
     const unsigned code = static_cast<unsigned>(as_int(misc[kMiscStatus]));
     const bool success = code == MR_STEP_SUCCESS;
-    // Capture + commit: a failed step publishes (and keeps) its checkpoint.
+    // Capture + commit: a failed step publishes (and keeps) its step-start
+    // state, which HBM still holds.
     float* qd = p.q + static_cast<size_t>(env) * nq;
     float* vd = p.v + static_cast<size_t>(env) * nv;
-    const float* qsrc = s + (success ? layout.q : layout.qc);
-    const float* vsrc = s + (success ? layout.v : layout.vc);
+    const float* qsrc = success ? s + layout.q : srcq;
+    const float* vsrc = success ? s + layout.v : srcv;
     float* obs = p.observations ? p.observations + static_cast<size_t>(item) * (nq + nv) : nullptr;
 #pragma unroll 1
     for (int i = lane; i < nq; i += 32) {
