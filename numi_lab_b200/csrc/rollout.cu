@@ -698,6 +698,8 @@ struct MRTaskRolloutHandle {
             const std::uint32_t o = static_cast<std::uint32_t>(static_cast<std::uint64_t>(envs) * c / nchains);
             const std::uint32_t n = static_cast<std::uint32_t>(static_cast<std::uint64_t>(envs) * (c + 1) / nchains) - o;
             cudaStream_t cs = nchains > 1 ? chain_stream[c] : s;
+            const int most = step_warps_per_block();
+            const int step_warps = nchains > 1 ? most : numi::control_step_spread_warps(static_cast<int>(n), most);
             for (std::uint32_t k = 0; k < steps; ++k) {
                 if (tasked) check(numi::launch_task_observe(task_params(k, o, n, actions, masks, obs, status), cs), "task observe launch");
                 if (driven) enqueue_policy(k, o, n, const_cast<float*>(actions) + static_cast<size_t>(k) * envs * na, true, cs);
@@ -725,7 +727,7 @@ struct MRTaskRolloutHandle {
                 p.q_comp = precision == MR_PRECISION_COMPENSATED ? d_qcomp.ptr + static_cast<size_t>(o) * model.world.nq : nullptr;
                 p.audit = audit ? d_audit.ptr + static_cast<size_t>(o) * numi::kAuditWords : nullptr;
                 p.quality = quality_cfg;
-                check(numi::launch_control_step(p, step_layout(), contact, precision, quality, step_warps_per_block(), cs),
+                check(numi::launch_control_step(p, step_layout(), contact, precision, quality, step_warps, cs),
                       "control step launch");
                 if (audit)
                     check(numi::launch_audit_step(p, step_layout(), precision != MR_PRECISION_FP32, step_warps_per_block(), cs),

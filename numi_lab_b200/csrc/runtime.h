@@ -32,6 +32,9 @@ cudaError_t configure_control_step_kernels(size_t max_dynamic_smem);
 cudaError_t launch_audit_step(const StepParams& p, const WarpLayout& layout, bool fp64_inertia, int warps_per_block,
                               cudaStream_t stream);
 size_t control_step_table_bytes();
+// Environments per CTA, at most `most`, of a launch over `env_count`
+// environments that has the device to itself.
+int control_step_spread_warps(int env_count, int most);
 // Largest CTA (in warps) the control-step instance for (precision, quality) is built for.
 int control_step_max_warps_per_block(std::uint32_t precision, bool quality);
 
