@@ -1911,7 +1911,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
             const int my_depth = mine ? T.depth[lane] : -1;
             const int par = (mine && lane > 0) ? T.parent[lane] : lane;
             float3 dw = f3(0.0f, 0.0f, 0.0f), dv = f3(0.0f, 0.0f, 0.0f);
-            const float lkk = mine && lane > 0 && bc.dof >= 0 ? static_cast<float>(sqrt(st.D)) : 1.0f;  // as written by the ABA
+            const float inv = mine && lane > 0 && bc.dof >= 0 ? static_cast<float>(R(1) / sqrt(st.D)) : 0.0f;  // 1 / L_kk
             if (lane == 0 && T.floating) {
                 float xr[6];
 #pragma unroll
@@ -1938,7 +1938,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
                         const int k = bc.dof;
                         const float sum = static_cast<float>(st.U[0] * dw.x + st.U[1] * dw.y + st.U[2] * dw.z +
                                                              st.U[3] * dv.x + st.U[4] * dv.y + st.U[5] * dv.z);
-                        const float xk = (z[k] - sum / lkk) / lkk;
+                        const float xk = (z[k] - sum * inv) * inv;
                         v[k] += xk;
                         dw = dw + f3(st.s[0], st.s[1], st.s[2]) * xk;
                         dv = dv + f3(st.s[3], st.s[4], st.s[5]) * xk;
