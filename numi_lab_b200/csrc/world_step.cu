@@ -3,6 +3,7 @@
 #include "world_step.cuh"
 
 #include <algorithm>
+#include <cstdlib>
 #include <type_traits>
 
 namespace numi {
@@ -98,6 +99,7 @@ int control_step_max_warps_per_block(std::uint32_t precision, bool quality) {
 // 2048 environments beside another chain of 2048 take 4227 us in 147 CTAs of
 // 14 and 3670 us in 128 of 16.
 int control_step_spread_warps(int env_count, int most) {
+    if (std::getenv("NUMI_B200_STEP_WARPS_PER_BLOCK")) return most;  // the caller fixed it
     int device = 0, sms = 0;
     if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1)
