@@ -1,5 +1,5 @@
-"""The free-body kernel's launch shapes (warps per environment, shared memory)
-follow the body count and the environment count; no arithmetic does.  The
+"""Launch shapes follow the environment count (and, for free bodies, the body
+count: warps per environment, shared memory); no arithmetic does.  The
 first environments of a large world therefore end on the same bits as the
 same environments in a small one, on both sides of every rule, and also when
 a substep's contacts do not fit the small shape's shared memory."""
@@ -68,3 +68,25 @@ def test_contacts_beyond_the_shared_arrays(cuda_device):
             assert (out["status"] == 0).all() and out["contacts"].min() > 126
             results.append(tuple(x[:FEW] for x in w.state()))
     _same(*results)
+
+
+# Environments per CTA of the articulated kernel: one up to eight per SM (1184),
+# one CTA per SM up to a resident wave, then chains of full CTAs.
+@pytest.mark.parametrize("source,envs", [("tree29", 1184), ("tree29", 1190), ("tree29", 2400), ("chain7", 1190)])
+def test_articulated_launches_give_the_same_bits(cuda_device, source, envs):
+    import torch
+
+    options = {"substeps": 1, "control_dt": 0.005} if source == "chain7" else {"substeps": 4, "velocity_iterations": 8, "control_dt": 0.02}
+    ends = []
+    for n in (FEW, envs):
+        with nb.World(source, n, seed=5, **options) as w:
+            gen = np.random.default_rng(3)
+            acts = gen.normal(0.0, 0.3, (10, FEW, w.action_count)).astype(np.float32)
+            acts = np.tile(acts, (1, -(-n // FEW), 1))[:, :n]
+            q, v, _ = nb.sample_reset(source, 5, 5, 0, FEW)
+            w.set_state(np.tile(q, (-(-n // FEW), 1))[:n], np.tile(v, (-(-n // FEW), 1))[:n])
+            _, status, _ = w.step(torch.from_numpy(np.ascontiguousarray(acts)).cuda(), wait=True)
+            assert int(status.abs().sum()) == 0
+            q1, v1, m = w.state()
+            ends.append((q1[:FEW], v1[:FEW], np.frombuffer(bytes(m), np.uint8)[:FEW * w.pair_count * 224]))
+    _same(*ends)
