@@ -57,14 +57,16 @@ __device__ __forceinline__ bool qnormalize(float4 in, float4& out, bool require_
     return finite4(out);
 }
 
-// Normalises a product of unit quaternions.  Near one, 1 / |q| is its Taylor
-// polynomial in |q|^2 - 1 (the next term, 5/16 (1e-3)^3, is below FP32
-// rounding): no square root or division on the way down a kinematic chain.
-__device__ __forceinline__ bool qrenormalize(float4 in, float4& out) {
-    const float d = qdot(in, in) - 1.0f;
-    if (!(fabsf(d) <= 1.0e-3f)) return qnormalize(in, out, false);
-    out = qscale(in, fmaf(d, fmaf(d, 0.375f, -0.5f), 1.0f));
-    return true;
+// Normalises a body's orientation on the way down a kinematic chain.  The
+// roundings of the squared norm are spelled out: which product a contraction
+// leaves rounded would otherwise depend on the code around it, and one ulp
+// here is what makes a contact world take another contact decision.
+__device__ __forceinline__ bool qnormalize_chain(float4 in, float4& out) {
+    if (!finite4(in)) return false;
+    const float n2 = __fmaf_rn(in.w, in.w, __fmaf_rn(in.z, in.z, __fmaf_rn(in.y, in.y, __fmul_rn(in.x, in.x))));
+    if (!(n2 > 1.0e-12f) || !isfinite(n2)) return false;
+    out = qscale(in, 1.0f / sqrtf(n2));
+    return finite4(out);
 }
 
 // Exponential-map increment for a world angular displacement h*omega,

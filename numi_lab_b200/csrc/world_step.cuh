@@ -234,14 +234,14 @@ __device__ __forceinline__ void body_inertia(const DeviceModel& M, int b, float4
 // ---------------------------------------------------------------------------
 // Forward kinematics (ArticulatedABA.metal:735-905): lane b owns body b.
 // Only what a body needs from its parent goes level by level, by warp
-// shuffle from the parent's lane: the orientation (one quaternion product
-// with the joint's own transform), then position and twist (a rotated offset
-// and one cross product).  The joint transforms, the rotated anchors and
-// axes, and the bias accelerations are computed by all lanes at once around
-// those two sweeps, because a level keeps at most a few lanes busy.  Leaves
-// the pose in shared memory (for collision) and the joint axis / origin of
-// the body's DoF in the Jacobian table; bias accelerations, offset and
-// subspace stay in registers.
+// shuffle from the parent's lane: the orientation, then position and twist.
+// Joint motions, rotated anchors and axes, and the bias accelerations are
+// computed by all lanes at once around those two sweeps, because a level
+// keeps at most a few lanes busy.  Every expression is the one a single
+// sweep evaluates, so the split changes no bit of a pose, twist or bias.
+// Leaves the pose in shared memory (for collision) and the joint axis /
+// origin of the body's DoF in the Jacobian table; bias accelerations, offset
+// and subspace stay in registers.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float3 shfl3(float3 a, int src) {
     return f3(__shfl_sync(0xffffffffu, a.x, src), __shfl_sync(0xffffffffu, a.y, src), __shfl_sync(0xffffffffu, a.z, src));
@@ -303,64 +303,65 @@ __device__ void kinematics(const Warp& w, const BodyConst& bc, BodyState<R>& st)
     const bool prismatic = child && bc.type == MR_JOINT_PRISMATIC;
     const bool turns = has && !prismatic;
     const float3 zero = f3(0.0f, 0.0f, 0.0f);
-    // Joint transform in the parent's frame.
-    float4 local = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+    // Joint constants and motion.
+    float4 pr = make_float4(0.0f, 0.0f, 0.0f, 1.0f), cr = pr, motion = pr, pj = pr;
     float3 axis = zero, anchor = zero;
-    float qdj = 0.0f;
+    float qj = 0.0f, qdj = 0.0f;
     if (child) {
-        const float4 pr = M.parent_rotation[b];
-        const float3 unit = xyz(M.axis[b]);
-        axis = qrot(pr, unit);
+        pr = M.parent_rotation[b];
+        cr = M.child_rotation_conj[b];
+        axis = xyz(M.axis[b]);
         anchor = xyz(M.parent_anchor[b]);
-        local = pr;
         if (has) {
-            const float qj = q[bc.qidx];
+            qj = q[bc.qidx];
             qdj = v[bc.dof];
             if (turns) {
                 float sh, ch;
                 sincosf(0.5f * qj, &sh, &ch);
-                local = qmul(pr, make_float4(unit.x * sh, unit.y * sh, unit.z * sh, ch));
-            } else {
-                anchor = anchor + axis * qj;
+                motion = make_float4(axis.x * sh, axis.y * sh, axis.z * sh, ch);
             }
         }
-        local = qmul(local, M.child_rotation_conj[b]);
     }
 #pragma unroll 1
     for (int l = 1; l <= T.n_levels; ++l) {
         const float4 qp = shfl4(st.qr, par);
-        if (my_depth == l && !qrenormalize(qmul(qp, local), st.qr)) {
-            set_status(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(b));
-            st.qr = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+        if (my_depth == l) {
+            pj = qmul(qp, pr);
+            if (!qnormalize_chain(qmul(qmul(pj, motion), cr), st.qr)) {
+                set_status(misc, MR_STEP_NONFINITE_RESULT, static_cast<unsigned>(b));
+                st.qr = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+            }
         }
     }
     const float4 qp = shfl4(st.qr, par);
-    const float3 ja = qrot(qp, axis);
-    const float3 ptj = qrot(qp, anchor);  // parent COM -> joint
+    const float3 ja = qrot(pj, axis);
+    const float3 pa = qrot(qp, anchor);
     const float3 ca = child ? qrot(st.qr, xyz(M.child_anchor[b])) : zero;
     const float3 rate = ja * qdj;
-    const float3 dw = turns ? rate : zero;
-    const float3 dv = prismatic ? rate : -cross3(dw, ca);
-    if (child) st.r = ptj - ca;
 #pragma unroll 1
     for (int l = 1; l <= T.n_levels; ++l) {
         const float3 cp = shfl3(st.c, par);
         const float3 wp = shfl3(st.w, par);
         const float3 vp = shfl3(st.v, par);
         if (my_depth == l) {
-            st.c = cp + st.r;
-            st.w = wp + dw;
-            st.v = vp + cross3(wp, st.r) + dv;
+            float3 jp = cp + pa;
+            if (prismatic) jp = jp + ja * qj;
+            st.c = jp - ca;
+            st.w = wp + (turns ? rate : zero);
+            st.v = vp + cross3(wp, jp - cp) + (prismatic ? rate : zero) - cross3(st.w, ca);
         }
     }
     const float3 cp = shfl3(st.c, par);
     const float3 wp = shfl3(st.w, par);
     if (child) {
-        const float3 jp = cp + ptj;
+        float3 jp = cp + pa;
+        if (prismatic) jp = jp + ja * qj;
+        const float3 ptj = jp - cp;
         const float3 ml = prismatic ? ja : (has ? -cross3(ja, ca) : zero);
-        if (turns) st.ba = cross3(wp, rate);
-        const float3 pc = prismatic ? 2.0f * cross3(wp, rate) : zero;
+        if (turns) st.ba = cross3(wp, ja) * qdj;
+        const float3 pc = prismatic ? cross3(wp, ja) * (2.0f * qdj) : zero;
         st.bl = cross3(wp, cross3(wp, ptj)) + pc - cross3(st.ba, ca) - cross3(st.w, cross3(st.w, ca));
+        st.r = st.c - cp;
         if (turns) { st.s[0] = ja.x; st.s[1] = ja.y; st.s[2] = ja.z; }
         st.s[3] = ml.x; st.s[4] = ml.y; st.s[5] = ml.z;
         if (has) {
@@ -2085,7 +2086,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
             const int my_depth = mine ? T.depth[lane] : -1;
             const int par = (mine && lane > 0) ? T.parent[lane] : lane;
             float3 dw = f3(0.0f, 0.0f, 0.0f), dv = f3(0.0f, 0.0f, 0.0f);
-            const float inv = mine && lane > 0 && bc.dof >= 0 ? static_cast<float>(R(1) / sqrt(st.D)) : 0.0f;  // 1 / L_kk
+            const float lkk = mine && lane > 0 && bc.dof >= 0 ? static_cast<float>(sqrt(st.D)) : 1.0f;  // as written by the ABA
             if (lane == 0 && T.floating) {
                 float xr[6];
 #pragma unroll
@@ -2112,7 +2113,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
                         const int k = bc.dof;
                         const float sum = static_cast<float>(st.U[0] * dw.x + st.U[1] * dw.y + st.U[2] * dw.z +
                                                              st.U[3] * dv.x + st.U[4] * dv.y + st.U[5] * dv.z);
-                        const float xk = (z[k] - sum * inv) * inv;
+                        const float xk = (z[k] - sum / lkk) / lkk;
                         v[k] += xk;
                         dw = dw + f3(st.s[0], st.s[1], st.s[2]) * xk;
                         dv = dv + f3(st.s[3], st.s[4], st.s[5]) * xk;
