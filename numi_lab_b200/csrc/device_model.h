@@ -44,14 +44,8 @@ struct alignas(16) DeviceTables {
     // Factor rows hold only their ancestors: row k starts here, its entry t
     // belongs to the t-th ancestor DoF and its last entry is the diagonal.
     std::uint16_t row_start[kMaxDofs];
-    std::uint16_t factor_words;
-    // Bodies by tree depth: level l holds level_body[level_first[l]] up to
-    // level_body[level_first[l + 1]].
-    std::uint8_t level_first[kMaxBodies + 2];
-    std::uint8_t level_body[kMaxBodies];
-    std::uint8_t pad1[12];
+    std::uint16_t factor_words, reserved1[7];
 };
-static_assert(sizeof(DeviceTables) % 16 == 0, "copied by 16-byte words");
 
 struct alignas(16) DeviceModel {
     DeviceTables tables;

@@ -41,13 +41,6 @@ constexpr int kPoseStride = 7;                    // COM position (3), orientati
 constexpr int kJStride = 7;                       // joint axis (3), origin (3), translation flag
 constexpr int kSlotStride = kManifoldWords + 1;   // manifold slot
 
-// Words of one body in the backward sweep by rows (world_step.cuh):
-// inputs -- world inertia (6), bias force (6), velocity-product acceleration
-// (6), joint subspace (6), offset to the parent (3), mass -- then its
-// shifted articulated inertia (21) and bias (6), U (6), D and u.
-constexpr int kAbaStride = 35;
-enum AbaWord : int { kAbInertia = 0, kAbBias = 6, kAbAcc = 12, kAbS = 18, kAbR = 24, kAbShifted = 0, kAbShiftedBias = 21, kAbU = 27, kAbD = 33, kAbu = 34 };
-
 struct WarpLayout {
     int body_pose, dof_J;
     int q, v, vf, tgt;
@@ -56,7 +49,6 @@ struct WarpLayout {
     int misc;
     int manifolds, contacts, G, L;
     int narrow;  // narrowphase scratch; aliases the contact records and rows
-    int aba;     // per-body words of the backward sweep by rows (worlds without contact)
     int qcomp;   // compensation terms of q's running sums (compensated precision only)
     int quality; // FP64 workspace of the quality solver (quality.cuh; quality-solver instances only)
     int total;   // floats per warp
@@ -107,10 +99,8 @@ __host__ __device__ inline WarpLayout make_layout(int nb, int nv, int nq, int np
         const int need = align4(narrow_words) - align4(ncap * kContactWords);
         L.G = take(rows > need ? rows : need);
         L.narrow = L.contacts;
-        L.aba = o;
     } else {
         L.manifolds = L.contacts = L.G = L.L = L.narrow = o;
-        L.aba = take(nb * kAbaStride);
     }
     L.qcomp = compensated ? take(nq) : o;
     L.quality = quality_doubles > 0 ? take(2 * quality_doubles) : o;

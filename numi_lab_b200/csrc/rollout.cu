@@ -229,13 +229,6 @@ numi::DeviceModel numi::rt::pack_model(const numi::CompiledModel& m, float h) {
             }
         }
         t.child_offsets[nb] = static_cast<std::uint8_t>(d.child_offsets[nb]);
-        int placed = 0;
-        for (std::uint32_t l = 0; l <= m.level_count; ++l) {
-            t.level_first[l] = static_cast<std::uint8_t>(placed);
-            for (int b = 0; b < nb; ++b)
-                if (depth[b] == static_cast<int>(l)) t.level_body[placed++] = static_cast<std::uint8_t>(b);
-        }
-        t.level_first[m.level_count + 1] = static_cast<std::uint8_t>(placed);
         std::uint16_t row = 0;
         for (std::uint32_t dof = 0; dof < w.nv; ++dof) {
             t.row_start[dof] = row;

@@ -33,9 +33,7 @@
 // instruction cache.  Loops whose body is more than a few instructions are
 // therefore rolled (`unroll 1`), or unrolled by two to four where their loads
 // are a chain.  4096 tree29 environments, four control steps: 270 KB of code
-// 6804 us, 207 KB 5598 us, the same bits.  With the two-sweep kinematics and
-// 14.1 KB instead of 16.9 KB of shared memory per environment (16 on an SM
-// instead of 13) they take 3733 us.
+// 6804 us, 207 KB 5598 us, the same bits.
 #pragma once
 
 #include "device_model.h"
@@ -47,7 +45,6 @@
 
 #include <cfloat>
 #include <cstdint>
-#include <type_traits>
 
 namespace numi {
 namespace {
@@ -382,140 +379,11 @@ __device__ void kinematics(const Warp& w, const BodyConst& bc, BodyState<R>& st)
 }
 
 // ---------------------------------------------------------------------------
-// Backward sweep of the ABA by rows, for FP32 worlds without contact: at most
-// a few bodies share a tree level, so six lanes take one body (five bodies at
-// a time), a row of its 6x6 inertia each, and the rank-one update and the
-// shift to the parent cost a lane six entries instead of thirty-six.  A
-// body's inputs, its shifted inertia for the parent, and U, D and u live in
-// its shared-memory words (AbaWord).  Sums over the six rows are taken in row
-// order by every lane, so all of them use the same bits.  Leaves the root's
-// summed inertia and bias in its words.  1024 seven-link chains, 20 steps:
-// 312 us lane by lane, 302 by rows, and the error against 64 bits falls from
-// 3.7e-6 to 3.2e-6 (geometric mean of eight seeds).  Contact worlds keep the
-// lane-per-body sweep: rows gave 4096 trees 3 %, but their longer chain of
-// shuffles cost a single environment 6 % and the converged solver 2 %.
-// ---------------------------------------------------------------------------
-__device__ void aba_backward_rows(const Warp& w, float* ab, const float* tau) {
-    const DeviceModel& M = *w.M;
-    const DeviceTables& T = *w.T;
-    float* misc = w.s + w.L->misc;
-    const int lane = w.lane;
-    const int g = lane / 6, i = lane - 6 * g, base = 6 * g;
-    int at[6];  // packed position of this row's entries
-#pragma unroll
-    for (int j = 0; j < 6; ++j) at[j] = sym6(i, j);
-    const bool angular = i < 3;
-    // Rows that E = [r]x mixes into angular row i, and r's entries there.
-    const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
-    const int j1 = (base + (angular ? 3 + i1 : i)) & 31, j2 = (base + (angular ? 3 + i2 : i)) & 31;
-#pragma unroll 1
-    for (int l = T.n_levels; l >= (T.floating ? 0 : 1); --l) {
-#pragma unroll 1
-        for (int first = T.level_first[l]; first < T.level_first[l + 1]; first += 5) {
-            const bool act = g < 5 && first + g < T.level_first[l + 1];
-            const int body = T.level_body[act ? first + g : first];
-            float* X = ab + body * kAbaStride;
-            float I[6];
-            const float mass = X[kAbD];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                I[j] = angular ? X[kAbInertia + at[j]] : 0.0f;
-                I[3 + j] = i == 3 + j ? mass : 0.0f;
-            }
-            float p = X[kAbBias + i];
-            const int c0 = T.child_offsets[body], children = T.child_offsets[body + 1] - c0;
-#pragma unroll 1
-            for (int k = 0; k < T.level_children[l]; ++k) {
-                if (k >= children) continue;
-                const float* Y = ab + T.children[c0 + k] * kAbaStride;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) I[j] += Y[kAbShifted + at[j]];
-                p += Y[kAbShiftedBias + i];
-            }
-            float U = 0.0f, D = 1.0f, u = 0.0f;
-            if (l > 0) {
-                float sv[6], Uj[6], qj[6];
-                float moved = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    sv[j] = X[kAbS + j];
-                    U = fmaf(I[j], sv[j], U);
-                    moved = fmaf(I[j], X[kAbAcc + j], moved);
-                }
-                p += moved;
-                float most = 0.0f;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) most = fmaxf(most, fabsf(I[j]));
-                most = fmaxf(most, __shfl_sync(0xffffffffu, most, (base + (i + 3) % 6) & 31));
-                most = fmaxf(most, __shfl_sync(0xffffffffu, most, (base + (i + 1) % 6) & 31));
-                most = fmaxf(most, __shfl_sync(0xffffffffu, most, (base + (i + 2) % 6) & 31));
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    Uj[j] = __shfl_sync(0xffffffffu, U, (base + j) & 31);
-                    qj[j] = __shfl_sync(0xffffffffu, p, (base + j) & 31);
-                }
-                const int dof = T.body_dof[body];
-                if (dof != kNone) {
-                    D = M.armature_eff[dof];
-                    u = tau[dof];
-#pragma unroll
-                    for (int j = 0; j < 6; ++j) {
-                        D = fmaf(sv[j], Uj[j], D);
-                        u = fmaf(-sv[j], qj[j], u);
-                    }
-                    const float floor = fmaxf(kAbsolutePivotFloor, most * 6.0f * kFloatEps);
-                    if (!(D > floor) || !isfinite(D)) {
-                        if (act && i == 0) set_status(misc, MR_STEP_FACTORIZATION_FAILED, static_cast<unsigned>(dof));
-                        D = 1.0f;
-                        u = 0.0f;
-                    } else {
-                        const float invD = 1.0f / D;
-                        const float scaled = U * invD;
-                        p = fmaf(U, u * invD, p);
-#pragma unroll
-                        for (int j = 0; j < 6; ++j) I[j] = fmaf(-scaled, Uj[j], I[j]);
-                    }
-                } else {
-                    U = 0.0f;
-                }
-                // X^T I X: angular columns of every row, then angular rows.
-                const float rx = X[kAbR], ry = X[kAbR + 1], rz = X[kAbR + 2];
-                I[0] -= I[4] * rz - I[5] * ry;
-                I[1] -= I[5] * rx - I[3] * rz;
-                I[2] -= I[3] * ry - I[4] * rx;
-                const float e1 = angular ? -X[kAbR + i2] : 0.0f, e2 = angular ? X[kAbR + i1] : 0.0f;
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    const float a = __shfl_sync(0xffffffffu, I[j], j1), b = __shfl_sync(0xffffffffu, I[j], j2);
-                    I[j] = fmaf(e1, a, fmaf(e2, b, I[j]));
-                }
-                const float p1 = __shfl_sync(0xffffffffu, p, j1), p2 = __shfl_sync(0xffffffffu, p, j2);
-                p = fmaf(e1, p1, fmaf(e2, p2, p));
-            }
-            __syncwarp();  // every lane has read the body's inputs
-            if (act) {
-#pragma unroll
-                for (int j = 0; j < 6; ++j)
-                    if (j <= i) X[kAbShifted + at[j]] = I[j];
-                X[kAbShiftedBias + i] = p;
-                X[kAbU + i] = U;
-                if (i == 0) {
-                    X[kAbD] = D;
-                    X[kAbu] = u;
-                }
-            }
-            __syncwarp();
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Articulated-body algorithm (ArticulatedABA.metal:905-1440): per-body COM
-// frames in world axes, classical accelerations, 21-entry inertias.  kRows
-// sweeps backward by rows (above), otherwise lane by lane: each body shifts
-// its articulated inertia and bias into its parent's frame in its own
-// registers; the parent pulls its children's contributions by warp shuffle in
-// a fixed order, so the sums are deterministic without atomics.
+// frames in world axes, classical accelerations, 21-entry inertias.  Each
+// body shifts its articulated inertia and bias into its parent's frame in
+// its own registers; the parent pulls its children's contributions by warp
+// shuffle in a fixed order, so the sums are deterministic without atomics.
 // With `factor` non-null (contact worlds) the body lanes also write their
 // rows of the joint-space factor H = L^T L (rows 0-5 of a floating root come
 // from the root's 6x6 factorisation): eliminating a DoF's descendants
@@ -525,7 +393,7 @@ __device__ void aba_backward_rows(const Warp& w, float* ab, const float* tau) {
 // contact body's list is its position in the rows of the DoFs below it, so
 // the substitution reads a row by consecutive words.
 // ---------------------------------------------------------------------------
-template <typename R, bool kRows>
+template <typename R>
 __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float* factor) {
     const DeviceModel& M = *w.M;
     const DeviceTables& T = *w.T;
@@ -549,7 +417,6 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
     kinematics(w, bc, st);
     if (!warp_ok(misc)) return false;
 
-    float* ab = s + L.aba;
     // Rigid inertia and velocity-dependent bias about the COM.
 #pragma unroll
     for (int e = 0; e < 21; ++e) st.I[e] = R(0);
@@ -570,25 +437,7 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
             bf = bf + md.y * st.v;
         }
         st.p[0] = bt.x; st.p[1] = bt.y; st.p[2] = bt.z; st.p[3] = bf.x; st.p[4] = bf.y; st.p[5] = bf.z;
-        if constexpr (kRows) {
-            float* X = ab + b * kAbaStride;
-            X[kAbInertia + 0] = Iw[0][0];
-            X[kAbInertia + 1] = Iw[1][0];
-            X[kAbInertia + 2] = Iw[1][1];
-            X[kAbInertia + 3] = Iw[2][0];
-            X[kAbInertia + 4] = Iw[2][1];
-            X[kAbInertia + 5] = Iw[2][2];
-#pragma unroll
-            for (int e = 0; e < 6; ++e) {
-                X[kAbBias + e] = st.p[e];
-                X[kAbS + e] = st.s[e];
-            }
-            st3(X + kAbAcc, st.ba);
-            st3(X + kAbAcc + 3, st.bl);
-            st3(X + kAbR, st.r);
-            X[kAbD] = md.x;
-        }
-        if (!kRows && b == 0 && T.floating) {
+        if (b == 0 && T.floating) {
             for (int k = 0; k < 3; ++k) {
                 st.I[sym6(3 + k, 3 + k)] += M.armature_eff[k];
                 st.I[sym6(k, k)] += M.armature_eff[3 + k];
@@ -603,34 +452,11 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
     const int first_child = mine ? T.child_offsets[b] : 0;
     const int n_children = mine ? T.child_offsets[b + 1] - first_child : 0;
     float3 acc_ang = f3(0.0f, 0.0f, 0.0f), acc_lin = f3(0.0f, 0.0f, 0.0f);
-    if constexpr (kRows) {
-        __syncwarp();
-        aba_backward_rows(w, ab, tau);
-        const float* X = ab + (mine ? b : 0) * kAbaStride;
-        if (mine && b > 0) {
-#pragma unroll
-            for (int e = 0; e < 6; ++e) st.U[e] = X[kAbU + e];
-            st.D = X[kAbD];
-            st.u = X[kAbu];
-        } else if (b == 0 && T.floating) {
-#pragma unroll
-            for (int e = 0; e < 21; ++e) st.I[e] = X[kAbShifted + e];
-#pragma unroll
-            for (int e = 0; e < 6; ++e) st.p[e] = X[kAbShiftedBias + e];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                st.I[sym6(3 + k, 3 + k)] += M.armature_eff[k];
-                st.I[sym6(k, k)] += M.armature_eff[3 + k];
-                st.p[k] -= tau[3 + k];
-                st.p[3 + k] -= tau[k];
-            }
-        }
-    }
 #pragma unroll 1
-    for (int l = kRows ? 0 : T.n_levels; l >= 0; --l) {
+    for (int l = T.n_levels; l >= 0; --l) {
         const bool active = my_depth == l;
 #pragma unroll 1
-        for (int k = 0; !kRows && k < T.level_children[l]; ++k) {
+        for (int k = 0; k < T.level_children[l]; ++k) {
             const bool take = active && k < n_children;
             const int src = take ? T.children[first_child + k] : b;
 #pragma unroll
@@ -645,7 +471,7 @@ __device__ bool aba(const Warp& w, const BodyConst& bc, BodyState<R>& st, float*
             }
         }
         if (!active) continue;
-        if (!kRows && l > 0) {
+        if (l > 0) {
             R prop[6];
             const float cv[6] = {st.ba.x, st.ba.y, st.ba.z, st.bl.x, st.bl.y, st.bl.z};
             sym6_mul(st.I, cv, prop);
@@ -2267,8 +2093,7 @@ __device__ __forceinline__ void control_step_item(const StepParams& p, const War
     for (int sub = 0; sub < p.substeps; ++sub) {
         compute_drives(w);
         __syncwarp();
-        constexpr bool kRows = !kContact && std::is_same<R, float>::value;
-        bool ok = aba<R, kRows>(w, bc, st, kContact ? s + layout.L : nullptr);
+        bool ok = aba(w, bc, st, kContact ? s + layout.L : nullptr);
         if (ok) {
             if (kContact)
                 ok = contact_substep<kComp, kQuality>(w, bc, st, sub + 1 == p.substeps, p.velocity_iterations,

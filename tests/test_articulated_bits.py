@@ -25,6 +25,8 @@ CASES = {
     "tree29_fp64_inertia": ("tree29", "fp64-inertia", None, 3),
     "tree29_compensated": ("tree29", "compensated", None, 3),
     "tree29_quality": ("tree29", "fp32", "quality_newton", 1),
+    "chain7_fp32": ("chain7", "fp32", None, 20),
+    "chain7_fp64_inertia": ("chain7", "fp64-inertia", None, 20),
 }
 
 
