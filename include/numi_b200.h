@@ -1184,9 +1184,10 @@ MR_API int mr_task_rollout_copy_environment_parameters(
     const MRTaskRolloutHandle* handle, float* friction_scale);
 
 /* No counterpart in the reference: the control-step kernel's launch shape
- * for the current precision mode (environments per CTA and resident
- * environments per SM, from the occupancy query at creation; 1 and 0 for
- * pile and stack worlds, whose kernel runs one environment per CTA). */
+ * in the current precision mode and solver: the environments per CTA that an
+ * advance launches, and the environments resident per SM in CTAs of that
+ * size (1 and 0 for pile and stack worlds, whose kernel runs one environment
+ * per CTA). */
 MR_API int mr_task_rollout_launch_shape(const MRTaskRolloutHandle* handle, uint32_t* warps_per_block,
                                         uint32_t* resident_warps_per_sm);
 /* No counterpart in the reference: how many environment chains an

@@ -632,7 +632,13 @@ struct MRTaskRolloutHandle {
         return precision == MR_PRECISION_COMPENSATED ? layout_comp : layout;
     }
     int step_warps_per_block() const { return quality ? warps_per_block_q[precision] : warps_per_block[precision]; }
-    int step_resident_warps_per_sm() const { return quality ? resident_warps_per_sm_q[precision] : resident_warps_per_sm[precision]; }
+    int chain_count() const { return static_cast<int>(std::min<std::uint32_t>(static_cast<std::uint32_t>(chains), envs)); }
+    // Environments per CTA that an articulated advance launches: chains share
+    // the device and keep the largest CTA.
+    int launch_warps() const {
+        const int most = step_warps_per_block();
+        return chain_count() > 1 ? most : numi::control_step_spread_warps(static_cast<int>(envs), most);
+    }
 
     size_t manifold_words() const {
         return scene ? static_cast<size_t>(numi::kSceneManifolds) * numi::kSceneSlotWords
@@ -689,7 +695,8 @@ struct MRTaskRolloutHandle {
         // With a policy each chain evaluates it on its own block before each
         // of its steps; with a task, observe runs before the policy, apply
         // after it and complete after the physics step.
-        const int nchains = static_cast<int>(std::min<std::uint32_t>(static_cast<std::uint32_t>(chains), envs));
+        const int nchains = chain_count();
+        const int step_warps = launch_warps();
         if (nchains > 1) {
             check(cudaEventRecord(ev_fork, s), "event");
             for (int c = 0; c < nchains; ++c) check(cudaStreamWaitEvent(chain_stream[c], ev_fork, 0), "stream wait");
@@ -698,8 +705,6 @@ struct MRTaskRolloutHandle {
             const std::uint32_t o = static_cast<std::uint32_t>(static_cast<std::uint64_t>(envs) * c / nchains);
             const std::uint32_t n = static_cast<std::uint32_t>(static_cast<std::uint64_t>(envs) * (c + 1) / nchains) - o;
             cudaStream_t cs = nchains > 1 ? chain_stream[c] : s;
-            const int most = step_warps_per_block();
-            const int step_warps = nchains > 1 ? most : numi::control_step_spread_warps(static_cast<int>(n), most);
             for (std::uint32_t k = 0; k < steps; ++k) {
                 if (tasked) check(numi::launch_task_observe(task_params(k, o, n, actions, masks, obs, status), cs), "task observe launch");
                 if (driven) enqueue_policy(k, o, n, const_cast<float*>(actions) + static_cast<size_t>(k) * envs * na, true, cs);
@@ -2071,15 +2076,24 @@ MR_API int mr_task_rollout_copy_environment_parameters(const MRTaskRolloutHandle
 MR_API uint32_t mr_task_rollout_environment_chains(const MRTaskRolloutHandle* handle) {
     if (!handle) return 0u;
     if (handle->scene) return 1u;
-    return static_cast<uint32_t>(std::min<std::uint32_t>(static_cast<std::uint32_t>(handle->chains), handle->envs));
+    return static_cast<uint32_t>(handle->chain_count());
 }
 
 MR_API int mr_task_rollout_launch_shape(const MRTaskRolloutHandle* handle, uint32_t* warps_per_block,
                                         uint32_t* resident_warps_per_sm) {
     return guarded([&] {
         if (!handle) throw std::invalid_argument("handle is null");
-        if (warps_per_block) *warps_per_block = handle->scene ? 1u : static_cast<uint32_t>(handle->step_warps_per_block());
-        if (resident_warps_per_sm) *resident_warps_per_sm = handle->scene ? 0u : static_cast<uint32_t>(handle->step_resident_warps_per_sm());
+        if (handle->scene) {
+            if (warps_per_block) *warps_per_block = 1u;
+            if (resident_warps_per_sm) *resident_warps_per_sm = 0u;
+            return;
+        }
+        const int warps = handle->launch_warps();
+        const size_t smem = numi::control_step_table_bytes() + static_cast<size_t>(handle->step_layout().total) * sizeof(float) * warps;
+        int blocks = 0;
+        check(numi::control_step_occupancy(handle->contact, handle->precision, handle->quality, warps, smem, &blocks), "occupancy query");
+        if (warps_per_block) *warps_per_block = static_cast<uint32_t>(warps);
+        if (resident_warps_per_sm) *resident_warps_per_sm = static_cast<uint32_t>(blocks * warps);
     });
 }
 

@@ -501,8 +501,9 @@ class World:
         return self._lib.lib.mr_task_rollout_layout(self._handle)
 
     def launch_shape(self) -> tuple[int, int]:
-        """(environments per CTA, resident environments per SM) of the
-        control-step kernel in the current precision mode."""
+        """(environments per CTA that an advance launches, environments
+        resident per SM in CTAs of that size) of the control-step kernel in
+        the current precision mode and solver."""
 
         wpb, res = ct.c_uint32(), ct.c_uint32()
         self._lib.check(self._lib.lib.mr_task_rollout_launch_shape(self._handle, ct.byref(wpb), ct.byref(res)), "launch_shape")

@@ -90,3 +90,27 @@ def test_articulated_launches_give_the_same_bits(cuda_device, source, envs):
             q1, v1, m = w.state()
             ends.append((q1[:FEW], v1[:FEW], np.frombuffer(bytes(m), np.uint8)[:FEW * w.pair_count * 224]))
     _same(*ends)
+
+
+def _sms():
+    import torch
+
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def _shape(envs, **options):
+    with nb.World("tree29", envs, substeps=4, velocity_iterations=8, control_dt=0.02, **options) as w:
+        return w.launch_shape()
+
+
+def test_the_reported_shape_is_the_launched_one(cuda_device):
+    """One environment per CTA up to eight per SM, then one CTA per SM up to
+    a resident wave, then two chains of full CTAs."""
+
+    sms = _sms()
+    full = 16  # environments per CTA and per SM at full residency
+    assert _shape(1)[0] == _shape(FEW)[0] == _shape(8 * sms)[0] == 1
+    assert _shape(8 * sms + 1) == (9, 9)
+    assert _shape(full * sms) == (full, full)
+    assert _shape(full * sms + 1) == (full, full)
+    assert _shape(FEW)[1] >= 8  # a spread launch is resident at once
