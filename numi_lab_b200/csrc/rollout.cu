@@ -288,6 +288,8 @@ void numi::rt::make_plan(const numi::CompiledModel& m, float h, KernelPlan& plan
     if (tables + static_cast<size_t>(plan.layout[0].total) * sizeof(float) > limit)
         throw std::runtime_error("per-environment shared memory exceeds the device limit");
     check(numi::configure_control_step_kernels(limit), "kernel attributes");
+    const char* fixed = std::getenv("NUMI_B200_STEP_WARPS_PER_BLOCK");
+    plan.spread = {fixed != nullptr, prop.multiProcessorCount};
     // Environments per CTA: the choice that keeps the most warps resident
     // per SM under the kernel's register and shared-memory footprint (each
     // CTA carries one copy of the topology tables).
@@ -299,7 +301,7 @@ void numi::rt::make_plan(const numi::CompiledModel& m, float h, KernelPlan& plan
             // what the instance is built for) instead of the search.
             const int max_wpb = numi::control_step_max_warps_per_block(prec, quality != 0);
             int lo = 1, hi = max_wpb;
-            if (const char* env = std::getenv("NUMI_B200_STEP_WARPS_PER_BLOCK")) lo = hi = std::max(1, std::min(max_wpb, std::atoi(env)));
+            if (fixed) lo = hi = std::max(1, std::min(max_wpb, std::atoi(fixed)));
             for (int wpb = lo; wpb <= hi; ++wpb) {
                 const size_t smem = tables + wpb * per_warp;
                 if (smem > limit) break;
@@ -442,6 +444,7 @@ struct MRTaskRolloutHandle {
     std::uint32_t precision = MR_PRECISION_FP32;  // MRPrecisionModeC
     int warps_per_block[numi::rt::kPrecisionModes] = {1, 1, 1};  // per precision mode
     int resident_warps_per_sm[numi::rt::kPrecisionModes] = {0, 0, 0};
+    numi::rt::SpreadRule spread{};
     MRTaskRolloutConfigC config{};
     std::uint32_t envs = 0;
     float h = 0.0f;
@@ -637,7 +640,7 @@ struct MRTaskRolloutHandle {
     // the device and keep the largest CTA.
     int launch_warps() const {
         const int most = step_warps_per_block();
-        return chain_count() > 1 ? most : numi::control_step_spread_warps(static_cast<int>(envs), most);
+        return chain_count() > 1 ? most : spread.warps(static_cast<int>(envs), most);
     }
 
     size_t manifold_words() const {
@@ -1065,6 +1068,7 @@ MR_API MRTaskRolloutHandle* mr_create_task_rollout(const MRRunManifestC* manifes
             numi::rt::KernelPlan plan;
             numi::rt::make_plan(h.model, h.h, plan);
             h.contact = plan.contact;
+            h.spread = plan.spread;
             h.dmodel = plan.dmodel;
             h.layout = plan.layout[0];
             h.layout_comp = plan.layout_comp[0];

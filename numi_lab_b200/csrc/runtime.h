@@ -32,9 +32,6 @@ cudaError_t configure_control_step_kernels(size_t max_dynamic_smem);
 cudaError_t launch_audit_step(const StepParams& p, const WarpLayout& layout, bool fp64_inertia, int warps_per_block,
                               cudaStream_t stream);
 size_t control_step_table_bytes();
-// Environments per CTA, at most `most`, of a launch over `env_count`
-// environments that has the device to itself.
-int control_step_spread_warps(int env_count, int most);
 // Largest CTA (in warps) the control-step instance for (precision, quality) is built for.
 int control_step_max_warps_per_block(std::uint32_t precision, bool quality);
 
@@ -98,11 +95,27 @@ int guarded(F&& f) {
     return -1;
 }
 
+// Environments per CTA, at most `most`, of a launch over `env_count`
+// environments that has the device to itself: one while that leaves at most
+// eight CTAs on an SM (each carries a copy of the topology tables), else one
+// CTA per SM.  1000 tree29 environments, four steps through the host call: 63
+// CTAs of 16 2032 us, 1000 of one 1663 us.  A launch that shares the device
+// keeps the largest CTA: 2048 environments beside another chain of 2048 take
+// 4227 us in 147 CTAs of 14 and 3670 us in 128 of 16.
+struct SpreadRule {
+    bool fixed = false;  // NUMI_B200_STEP_WARPS_PER_BLOCK was set when the plan was made
+    int sms = 1;         // of the plan's device
+    int warps(int env_count, int most) const {
+        if (fixed) return most;
+        const int per_sm = (env_count + sms - 1) / sms;
+        return per_sm <= 8 ? 1 : std::min(most, per_sm);
+    }
+};
+constexpr int kPrecisionModes = 3;       // indexed by MRPrecisionModeC
+constexpr int kSolverModes = 2;          // 0 temporalCone, 1 quality (contact worlds)
 // Everything the control-step kernel needs to know about a compiled model
 // at one substep length: the packed device record, the per-warp
 // shared-memory layout and the launch shape per (solver, precision mode).
-constexpr int kPrecisionModes = 3;       // indexed by MRPrecisionModeC
-constexpr int kSolverModes = 2;          // 0 temporalCone, 1 quality (contact worlds)
 struct KernelPlan {
     DeviceModel dmodel{};
     // [solver]: FP32 and FP64 articulated inertia; compensated adds the q
@@ -110,6 +123,7 @@ struct KernelPlan {
     WarpLayout layout[kSolverModes]{};
     WarpLayout layout_comp[kSolverModes]{};
     bool contact = false;
+    SpreadRule spread{};
     int warps_per_block[kSolverModes][kPrecisionModes] = {{1, 1, 1}, {1, 1, 1}};
     int resident_warps_per_sm[kSolverModes][kPrecisionModes] = {{0, 0, 0}, {0, 0, 0}};
     const WarpLayout& layout_for(std::uint32_t precision, bool quality = false) const {

@@ -395,7 +395,7 @@ struct MRServerHandle {
                 sp.velocity_iterations = static_cast<int>(config.velocity_iterations);
                 sp.final_velocity_iterations = static_cast<int>(config.final_velocity_iterations);
                 check(numi::launch_control_step(sp, p.plan.layout[0], p.plan.contact, MR_PRECISION_FP32, false,
-                                                numi::control_step_spread_warps(static_cast<int>(items), p.plan.warps_per_block[0][0]), p.stream),
+                                                p.plan.spread.warps(static_cast<int>(items), p.plan.warps_per_block[0][0]), p.stream),
                       "control step launch");
             }
             off += items;

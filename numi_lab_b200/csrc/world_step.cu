@@ -2,8 +2,6 @@
 // device code lives in world_step.cuh.
 #include "world_step.cuh"
 
-#include <algorithm>
-#include <cstdlib>
 #include <type_traits>
 
 namespace numi {
@@ -90,22 +88,6 @@ size_t control_step_table_bytes() { return sizeof(DeviceTables); }
 
 int control_step_max_warps_per_block(std::uint32_t precision, bool quality) {
     return precision == MR_PRECISION_FP32 && !quality ? kMaxStepWarpsPerBlock : 4;
-}
-
-// One environment per CTA while that leaves at most eight on an SM (each CTA
-// carries a copy of the topology tables), else one CTA per SM.  1000 tree29
-// environments, four steps through the host call: 63 CTAs of 16 2032 us,
-// 1000 of one 1663 us.  A launch that fills the device keeps the largest CTA:
-// 2048 environments beside another chain of 2048 take 4227 us in 147 CTAs of
-// 14 and 3670 us in 128 of 16.
-int control_step_spread_warps(int env_count, int most) {
-    if (std::getenv("NUMI_B200_STEP_WARPS_PER_BLOCK")) return most;  // the caller fixed it
-    int device = 0, sms = 0;
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1)
-        return most;
-    const int per_sm = (env_count + sms - 1) / sms;
-    return per_sm <= 8 ? 1 : std::min(most, per_sm);
 }
 
 namespace {

@@ -114,3 +114,15 @@ def test_the_reported_shape_is_the_launched_one(cuda_device):
     assert _shape(full * sms) == (full, full)
     assert _shape(full * sms + 1) == (full, full)
     assert _shape(FEW)[1] >= 8  # a spread launch is resident at once
+
+
+def test_a_fixed_cta_size_is_read_at_creation(cuda_device, monkeypatch):
+    options = {"substeps": 4, "velocity_iterations": 8, "control_dt": 0.02}
+    name = "NUMI_B200_STEP_WARPS_PER_BLOCK"
+    monkeypatch.delenv(name, raising=False)
+    with nb.World("tree29", FEW, **options) as spread:
+        monkeypatch.setenv(name, "4")
+        with nb.World("tree29", FEW, **options) as fixed:
+            assert (spread.launch_shape()[0], fixed.launch_shape()[0]) == (1, 4)
+            monkeypatch.delenv(name)
+            assert (spread.launch_shape()[0], fixed.launch_shape()[0]) == (1, 4)
