@@ -79,32 +79,49 @@ int scene_resident_limit() {
     return limit;
 }
 
+// SMs of the current device (0 when it cannot be asked).
+int device_sms() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms;
+}
+
 // Warps and shared memory (floats) of a launch over `envs` environments of
 // `nb` bodies.  The registers hold 16 warps per SM.  Four warps per
 // environment finish one soonest, so that is the shape while every
-// environment is resident at once (4 per SM); past that, fewer warps waste
-// less on barriers and idle lanes, and small worlds do best with one.
-// Measured, us per control step (start of the table: 1 / 2 / 4 warps):
-//   pile    9 bodies:  500 envs 229 / 216 / 205;  8000 envs 1246 / 1983 / 2565
-//   pile   20 bodies:  500 envs 318 / 239 / 213;  8000 envs 1852 / 2347 / 2947
-//   pile   36 bodies:  16384 envs 7292 / 6598 / 6813
-//   pile   47 bodies:  500 envs 652 / 374 / 278;  8000 envs 4368 / 3255 / 3612
-//   pile   61 bodies:  500 envs 837 / 527 / 362;  8000 envs 5243 / 4562 / 4695
+// environment is resident at once (4 per SM, 592 on 148 SMs); past that,
+// fewer warps waste less on barriers and idle lanes, and small worlds do best
+// with one.  us per control step of 1 / 2 / 4 warps (3370, 3370, 7000 floats
+// up to 28 bodies, 7000 above):
+//   pile    9 bodies:  592 envs 224 / 210 / 203;  4000 envs  610 /  983 / 1234
+//   pile   20 bodies:  592 envs 316 / 233 / 213;  4000 envs  841 / 1129 / 1377
+//   pile   28 bodies:  592 envs 426 / 311 / 222;  4000 envs 1228 / 1616 / 1450
+//   pile   36 bodies:  592 envs 533 / 351 / 246;  4000 envs 2201 / 1568 / 1599
+//   pile   61 bodies:  592 envs 807 / 501 / 371;  4000 envs 3285 / 2176 / 2286
 // Support-mapped worlds keep per-thread polytopes in local memory, which
-// wants the L1 more than residency: 49-body hull piles, 1500 envs, 864 / 944
-// / 694; 23-body cylinder piles, 3000 envs, 1009 / 1030 / 1222.
+// wants the L1 more than residency, so above 28 bodies they keep four warps
+// at any environment count and below, with one warp, 2800 floats:
+//   hulls  35 bodies:  592 envs 282 / 216 / 136;  4000 envs 1028 /  740 /  705
+//   hulls  61 bodies:  592 envs 488 / 373 / 225;  4000 envs 2177 / 1671 / 1668
+//   capsule-box pairs through GJK, 35 bodies:     4000 envs 2862 / 2072 / 1817
+//   hulls   9 bodies, 4000 envs, one warp in 2800 / 3370 floats 447 / 463
+//   cylinders 14 bodies, 3000 envs,                             751 / 913
+//   cylinders 23 bodies, 3000 envs,                            1914 / 2119
+// Where the line costs most: 20 to 28 support-mapped bodies just past eight
+// environments per SM, where two warps are up to a fifth faster than one
+// (cylinders 23 bodies, 1500 envs 1366 / 1115; hulls 28 bodies 534 / 444).
 // Shared memory: no more than a shape uses, because what it leaves is L1.
 SceneShape scene_shape(int nb, int envs, bool compensated, bool convex) {
     SceneShape shape{};
     constexpr int kSmall = 28;   // bodies
-    constexpr int kResidentFour = 4 * 148, kResidentTwo = 8 * 148;
+    const int sms = device_sms();
     int total = 7000;
-    if (envs <= kResidentFour || (convex && nb > kSmall)) {
+    if (envs <= 4 * sms || (convex && nb > kSmall)) {
         shape.warps = 4;
     } else if (nb > kSmall) {
         shape.warps = 2;
     } else {
-        shape.warps = envs <= kResidentTwo ? 2 : 1;
+        shape.warps = envs <= 8 * sms ? 2 : 1;
         total = convex && shape.warps == 1 ? 2800 : 3370;
     }
     const int words = std::max(kUnionLeast, std::min(kUnionMost, total - scene_smem_words(nb, 0, compensated)));
