@@ -110,6 +110,8 @@ struct SceneShape {
     int warps;
     size_t smem;
 };
+// Warps per environment that launch_scene_step takes for these parameters.
+int scene_step_warps(const SceneParams& p);
 // ... of the batch's free-body family, for any mix of worlds.
 int mix_scene_warps();
 size_t mix_scene_smem_bytes();

@@ -203,6 +203,8 @@ cudaError_t launch_scene_audit(const SceneParams& p, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
+int scene_step_warps(const SceneParams& p) { return scene_shape(p.bodies, p.env_count, p.q_comp != nullptr, p.support_mapped != 0).warps; }
+
 cudaError_t launch_scene_step(const SceneParams& p, cudaStream_t stream) {
     const bool compensated = p.q_comp != nullptr;
     if (p.bodies < 1 || p.bodies > kSceneMaxBodies) return cudaErrorInvalidValue;

@@ -325,9 +325,36 @@ struct MRServerHandle {
         p.admitted.clear();
     }
 
+    // The tick's pools share the device.  An articulated launch spreads over
+    // its SMs only while all their warps are resident at once (16 per SM by
+    // registers, in either kernel); past that it would hold SMs that the
+    // other pools need.  us per tick of two steps, full CTAs / spread: 1000
+    // trees 652 / 528; 300 trees and 300 piles 664 / 558; 1000 trees and 500
+    // piles 743 / 798; 300 trees, 300 chains and 1000 piles 717 / 766.
+    bool tick_fits() const {
+        std::size_t warps = 0;
+        int sms = 0;
+        for (const auto& kv : pools) {
+            const Pool& p = *kv.second;
+            std::size_t envs = 0;
+            for (const Request* r : p.active) envs += r->envs;
+            if (p.scene) {
+                numi::SceneParams sp{};
+                sp.bodies = p.smodel.nb;
+                sp.env_count = static_cast<int>(envs);
+                sp.support_mapped = p.smodel.support_mapped;
+                warps += envs * numi::scene_step_warps(sp);
+            } else {
+                warps += envs;
+                sms = p.plan.spread.sms;
+            }
+        }
+        return warps <= static_cast<std::size_t>(sms) * numi::kMaxStepWarpsPerBlock;
+    }
+
     // Up to steps_per_tick control steps of every active request of the
     // pool (a request stops at its horizon), one launch per step.
-    void launch(Pool& p) {
+    void launch(Pool& p, bool spread) {
         p.step_items.assign(steps_per_tick, 0);
         p.tick_env_steps = 0;
         if (p.active.empty()) return;
@@ -394,8 +421,9 @@ struct MRServerHandle {
                 sp.substeps = static_cast<int>(config.physics_substeps);
                 sp.velocity_iterations = static_cast<int>(config.velocity_iterations);
                 sp.final_velocity_iterations = static_cast<int>(config.final_velocity_iterations);
+                const int most = p.plan.warps_per_block[0][0];
                 check(numi::launch_control_step(sp, p.plan.layout[0], p.plan.contact, MR_PRECISION_FP32, false,
-                                                p.plan.spread.warps(static_cast<int>(items), p.plan.warps_per_block[0][0]), p.stream),
+                                                spread ? p.plan.spread.warps(static_cast<int>(items), most) : most, p.stream),
                       "control step launch");
             }
             off += items;
@@ -546,9 +574,10 @@ MR_API int mr_server_tick(MRServerHandle* server, uint32_t* active_requests, uin
             }
         }
         std::uint32_t reqs = 0, envs = 0;
+        const bool spread = server->tick_fits();
         for (auto& kv : server->pools) {
             server->scatter_admissions(*kv.second);
-            server->launch(*kv.second);
+            server->launch(*kv.second, spread);
             reqs += static_cast<std::uint32_t>(kv.second->active.size());
             envs += kv.second->tick_env_steps;
         }

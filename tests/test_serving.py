@@ -111,3 +111,22 @@ def test_pile_request_matches_a_rollout_alone_and_in_a_mix(cuda_device):
         q_w, v_w, _ = world.state()
     np.testing.assert_array_equal(q_w, q_alone)
     np.testing.assert_array_equal(v_w, v_alone)
+
+
+@pytest.mark.gpu
+def test_request_result_is_the_same_where_the_tick_does_not_fit_the_device(cuda_device):
+    """Trees spread over the SMs while the tick's warps are resident at once
+    (alone), and keep full CTAs beside more (600 piles of four warps)."""
+
+    seed, envs, horizon = 11, 5, 3
+    results = []
+    for piles in (0, 600):
+        with nb.Server(model_seed=seed, max_envs_per_source=1024) as server:
+            acts = (0.3 * np.random.default_rng(1).standard_normal((horizon, envs, server.action_count("tree29")))).astype(np.float32)
+            ids = [server.submit("pile", piles, horizon, 7, np.zeros((horizon, piles, 0), np.float32))] if piles else []
+            ids.append(server.submit("tree29", envs, horizon, seed, acts))
+            done = _run_until_done(server, ids)
+            assert all(done[i].failed_env_steps == 0 for i in ids)
+            results.append(server.result(ids[-1]))
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
