@@ -790,9 +790,10 @@ def measure_mix(args, device) -> dict:
                                f"{horizon} control steps per bench step", "worlds": len(worlds),
                    "l2": "flushed (256 MiB write) between steps"},
         "batch_launch": shape,
-        # Batched: the queue reset plus one persistent launch per horizon (fused)
-        # or one per device-code family; plain: one launch per world and step.
-        "gpu_launches_per_step": {"batched": 1 if shape["mode"] == 0 else 2, "plain_per_config": horizon * len(worlds)},
+        # Batched: the queue reset plus one persistent launch per horizon and
+        # device-code family; plain: one launch per world and step.
+        "gpu_launches_per_step": {"batched": (shape["blocks"] > 0) + (shape["scene_blocks"] > 0),
+                                  "plain_per_config": horizon * len(worlds)},
         "failed_env_steps": {"batched": batch_fail, "plain_per_config": plain_fail, "concurrent_streams": conc_fail},
     }
 

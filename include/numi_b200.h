@@ -1346,9 +1346,10 @@ enum MRBatchOrderC {
 };
 
 /* FUSED: one persistent launch runs every item (all worlds articulated).
- * PER_FAMILY: one per device-code family -- articulated, an environment per
- * warp, and free-body, an environment per CTA -- running concurrently, each
- * at its own kernel's register budget and occupancy. */
+ * PER_FAMILY (some world of free bodies): one per device-code family that
+ * the batch holds -- articulated, an environment per warp, and free-body, an
+ * environment per CTA -- running concurrently, each at its own kernel's
+ * register budget and occupancy. */
 enum MRBatchLaunchModeC {
     MR_BATCH_LAUNCH_FUSED = 0u,
     MR_BATCH_LAUNCH_PER_FAMILY = 1u
@@ -1357,7 +1358,7 @@ enum MRBatchLaunchModeC {
 typedef struct MRBatchLaunchShapeC {
     uint32_t worlds;
     uint32_t items;                  /* environments over all rollouts */
-    uint32_t warps_per_block;        /* articulated launch */
+    uint32_t warps_per_block;        /* articulated launch (these four: 0 without articulated worlds) */
     uint32_t blocks;                 /* persistent grid: SMs x resident CTAs */
     uint32_t resident_warps_per_sm;
     uint32_t shared_bytes_per_warp;
@@ -1365,7 +1366,7 @@ typedef struct MRBatchLaunchShapeC {
     uint32_t tuned;                  /* 1 after mr_batch_tune */
     float tuned_step_milliseconds;   /* the tuner's best time of one control step */
     uint32_t mode;                   /* MRBatchLaunchModeC */
-    uint32_t scene_blocks;           /* PER_FAMILY: the free-body launch's grid (one environment per CTA) */
+    uint32_t scene_blocks;           /* the free-body launch's grid, one environment per CTA (0 without free-body worlds) */
     uint32_t scene_resident_warps_per_sm;
 } MRBatchLaunchShapeC;
 
@@ -1383,10 +1384,9 @@ MR_API int mr_batch_advance(MRBatchHandle* batch, uint32_t control_step_count, c
                             const uint32_t* const* reset_masks, uint32_t* const* status_codes, uint64_t cuda_stream);
 /* No counterpart in the reference.  Autotuner: measures each rollout's item
  * latency (a launch of its environments alone), orders the queue by it,
- * then times control_step_count steps of the whole batch for both launch
- * modes, 1, 2 and 4 warps per CTA and both claim orders and keeps the
- * fastest.  Steps the
- * rollouts with `actions` (as in mr_batch_advance) and restores their
+ * then times control_step_count steps of the whole batch for both claim
+ * orders and, with articulated worlds, 1, 2 and 4 of their warps per CTA,
+ * and keeps the fastest.  Steps the rollouts with `actions` (as in mr_batch_advance) and restores their
  * state afterwards; synchronous. */
 MR_API int mr_batch_tune(MRBatchHandle* batch, uint32_t control_step_count, const float* const* actions);
 MR_API int mr_batch_launch_shape(const MRBatchHandle* batch, MRBatchLaunchShapeC* out);

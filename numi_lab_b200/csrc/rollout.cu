@@ -2471,6 +2471,7 @@ struct MRBatchHandle {
         std::uint32_t best_order = order;
         for (const std::uint32_t ord : {std::uint32_t(MR_BATCH_ORDER_LONGEST_FIRST), std::uint32_t(MR_BATCH_ORDER_ROUND_ROBIN)})
             for (const int wp : {1, 2, 4}) {
+                if (items[numi::kMixFamilyArticulated].empty() && wp != best_wpb) continue;  // no launch takes it
                 order = ord;
                 warps_per_block = wp;
                 try {
@@ -2586,15 +2587,17 @@ MR_API int mr_batch_launch_shape(const MRBatchHandle* batch, MRBatchLaunchShapeC
         *out = MRBatchLaunchShapeC{};
         out->worlds = static_cast<uint32_t>(batch->worlds.size());
         out->items = batch->item_count();
-        const int main_family = numi::kMixFamilyArticulated;
-        out->warps_per_block = static_cast<uint32_t>(batch->warps_per_block);
-        out->blocks = static_cast<uint32_t>(batch->grid(main_family));
-        out->resident_warps_per_sm = static_cast<uint32_t>(batch->blocks_per_sm[main_family] * batch->warps_per_block);
-        out->shared_bytes_per_warp = static_cast<uint32_t>(batch->smem_floats[main_family] * sizeof(float));
-        out->scene_blocks = batch->mode == MR_BATCH_LAUNCH_PER_FAMILY ? static_cast<uint32_t>(batch->grid(numi::kMixFamilyScene)) : 0u;
-        out->scene_resident_warps_per_sm =
-            batch->mode == MR_BATCH_LAUNCH_PER_FAMILY
-                ? static_cast<uint32_t>(batch->blocks_per_sm[numi::kMixFamilyScene] * numi::mix_scene_warps()) : 0u;
+        constexpr int art = numi::kMixFamilyArticulated, scn = numi::kMixFamilyScene;
+        if (!batch->items[art].empty()) {
+            out->warps_per_block = static_cast<uint32_t>(batch->warps_per_block);
+            out->blocks = static_cast<uint32_t>(batch->grid(art));
+            out->resident_warps_per_sm = static_cast<uint32_t>(batch->blocks_per_sm[art] * batch->warps_per_block);
+            out->shared_bytes_per_warp = static_cast<uint32_t>(batch->smem_floats[art] * sizeof(float));
+        }
+        if (!batch->items[scn].empty()) {
+            out->scene_blocks = static_cast<uint32_t>(batch->grid(scn));
+            out->scene_resident_warps_per_sm = static_cast<uint32_t>(batch->blocks_per_sm[scn] * numi::mix_scene_warps());
+        }
         out->mode = batch->mode;
         out->order = batch->order;
         out->tuned = batch->tuned ? 1u : 0u;

@@ -102,6 +102,26 @@ def test_tuned_batch_still_matches(cuda_device):
             w.close()
 
 
+@pytest.mark.parametrize("sources", [("chain7",), ("pile",), ("chain7", "pile")])
+def test_launch_shape_names_the_launches_that_run(cuda_device, sources):
+    options = {"chain7": {"substeps": 1, "control_dt": 0.005}, "pile": {"substeps": 4, "velocity_iterations": 8, "control_dt": 0.02}}
+    worlds = [nb.World(s, 5, **options[s]) for s in sources]
+    try:
+        with nb.Batch(worlds) as batch:
+            for tuned in (0, 1):
+                shape = batch.launch_shape()
+                articulated, free = "chain7" in sources, "pile" in sources
+                assert shape["tuned"] == tuned and shape["mode"] == (1 if free else 0) and shape["items"] == 5 * len(sources)
+                for name in ("warps_per_block", "blocks", "resident_warps_per_sm", "shared_bytes_per_warp"):
+                    assert (shape[name] > 0) == articulated, name
+                for name in ("scene_blocks", "scene_resident_warps_per_sm"):
+                    assert (shape[name] > 0) == free, name
+                batch.tune(_actions(worlds, 2, 3))
+    finally:
+        for w in worlds:
+            w.close()
+
+
 def test_batch_rejects_what_it_cannot_run(cuda_device):
     with nb.World("tree29", 4, precision="fp64-inertia") as w64, nb.World("chain7", 4, substeps=1, control_dt=0.005) as c:
         with pytest.raises(nb.MetalRoboError, match="FP32"):
