@@ -1099,8 +1099,10 @@ MR_API MRTaskRolloutHandle* mr_create_task_rollout(const MRRunManifestC* manifes
             }
         }
         // Two chains once the batch exceeds one resident wave of the FP32
-        // kernel (at 4096 tree29 envs: 2.3 waves; measured +18 % over one
-        // chain, three and four chains slower); NUMI_B200_CHAINS overrides.
+        // kernel.  us per control step of one / two chains: 2368 tree29
+        // environments (one wave) 599 / 595, 2400 767 / 658, 4096 (1.7 waves)
+        // 1111 / 1000, 16384 4044 / 3971; three and four chains are within
+        // three percent of two.  NUMI_B200_CHAINS overrides.
         if (!h.scene) {
             const long resident = static_cast<long>(h.resident_warps_per_sm[0]) * prop.multiProcessorCount;
             h.chains = static_cast<long>(h.envs) > resident ? 2 : 1;

@@ -1630,7 +1630,7 @@ struct ContactRow {
     float3 lambda;
     float pre[9];
 };
-// Rows past the first per thread, word-major in the workspace.
+// Rows past kOwnRows per thread, word-major in the workspace.
 __device__ __forceinline__ void store_row(float* R, int c, const ContactRow& r) {
     const float w[kRowWords] = {r.n.x, r.n.y, r.n.z, r.t.x, r.t.y, r.t.z, r.bt.x, r.bt.y, r.bt.z, r.target, r.reg, r.mu, r.relax,
                                 r.lambda.x, r.lambda.y, r.lambda.z, r.pre[0], r.pre[1], r.pre[2], r.pre[3], r.pre[4], r.pre[5],
@@ -1660,9 +1660,10 @@ __device__ __forceinline__ void store_lambda(float* R, int c, float3 l) {
 }
 
 // One CTA advances work item `item` of environment slot `env` by one control
-// step, with `s` its scene_step_smem_bytes() of shared memory.  Every thread
-// of the CTA calls it; it returns with the CTA synchronised on entry to the
-// commit but not after it.  kComp: compensated sums for positions (across
+// step, with `s` its dynamic shared memory (at least scene_smem_words() of a
+// union of kUnionLeast; what the launch gave more goes to the union).  Every
+// thread of the CTA calls it; it returns with the CTA synchronised on entry to
+// the commit but not after it.  kComp: compensated sums for positions (across
 // control steps, through p.q_comp) and for the velocity increments of the
 // sweeps.  kConvex: the world has support-mapped pairs.
 //

@@ -28,12 +28,14 @@
 // in generalized velocities (MetalWorldContact.metal:6655-7000), evaluated
 // without dense response columns.
 //
-// Instruction fetch bounds this kernel as much as issue does: 13 warps per SM
-// each sit at their own stage, so its whole code is the working set of the
-// instruction cache.  Loops whose body is more than a few instructions are
+// Instruction fetch bounds this kernel as much as issue does: the 16 warps of
+// an SM each sit at their own stage, so its whole code is the working set of
+// the instruction cache.  Loops whose body is more than a few instructions are
 // therefore rolled (`unroll 1`), or unrolled by two to four where their loads
 // are a chain.  4096 tree29 environments, four control steps: 270 KB of code
-// 6804 us, 207 KB 5598 us, the same bits.
+// 6804 us, 207 KB 5598 us; with the two-sweep kinematics and 14.1 KB instead
+// of 16.9 KB of shared memory per environment (16 on an SM instead of 13)
+// 4057 us; the same bits throughout.
 #pragma once
 
 #include "device_model.h"
@@ -1928,8 +1930,7 @@ __device__ bool contact_substep(const Warp& w, const BodyConst& bc, BodyState<R>
                 dw = f3(xr[3], xr[4], xr[5]);
             }
 #pragma unroll 1
-        #pragma unroll 1
-    for (int l = 1; l <= T.n_levels; ++l) {
+            for (int l = 1; l <= T.n_levels; ++l) {
                 const float3 pw = shfl3(dw, par);
                 const float3 pv = shfl3(dv, par);
                 if (my_depth == l) {
