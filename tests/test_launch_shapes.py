@@ -70,18 +70,29 @@ def test_contacts_beyond_the_shared_arrays(cuda_device):
     _same(*results)
 
 
-# Environments per CTA of the articulated kernel: one up to eight per SM (1184),
-# one CTA per SM up to a resident wave, then chains of full CTAs.
-@pytest.mark.parametrize("source,envs", [("tree29", 1184), ("tree29", 1190), ("tree29", 2400), ("chain7", 1190)])
-def test_articulated_launches_give_the_same_bits(cuda_device, source, envs):
+# Environments per CTA of the articulated kernel against one (a few
+# environments): one CTA per SM past eight environments on each (1184), full
+# CTAs of one resident wave and of two chains, the quality instance's three,
+# and four, by the override, where the plan itself holds one.
+@pytest.mark.parametrize("source,envs,precision,solver,per_cta,fixed", [
+    ("tree29", 1190, "fp32", None, 9, False), ("tree29", 2368, "fp32", None, 16, False), ("tree29", 2400, "fp32", None, 16, False),
+    ("tree29", 1190, "fp32", "quality_newton", 3, False), ("tree29", 1190, "fp64-inertia", None, 4, True),
+    ("tree29", 1190, "compensated", None, 4, True), ("chain7", 1190, "fp32", None, 4, True)])
+def test_articulated_launches_give_the_same_bits(cuda_device, monkeypatch, source, envs, precision, solver, per_cta, fixed):
     import torch
 
     options = {"substeps": 1, "control_dt": 0.005} if source == "chain7" else {"substeps": 4, "velocity_iterations": 8, "control_dt": 0.02}
+    steps = 2 if solver else 10
     ends = []
     for n in (FEW, envs):
-        with nb.World(source, n, seed=5, **options) as w:
+        if fixed and n == envs:
+            monkeypatch.setenv("NUMI_B200_STEP_WARPS_PER_BLOCK", str(per_cta))
+        with nb.World(source, n, seed=5, precision=precision, **options) as w:
+            if solver:
+                w.set_solver(solver)
+            assert w.launch_shape()[0] == (1 if n == FEW else per_cta)
             gen = np.random.default_rng(3)
-            acts = gen.normal(0.0, 0.3, (10, FEW, w.action_count)).astype(np.float32)
+            acts = gen.normal(0.0, 0.3, (steps, FEW, w.action_count)).astype(np.float32)
             acts = np.tile(acts, (1, -(-n // FEW), 1))[:, :n]
             q, v, _ = nb.sample_reset(source, 5, 5, 0, FEW)
             w.set_state(np.tile(q, (-(-n // FEW), 1))[:n], np.tile(v, (-(-n // FEW), 1))[:n])
