@@ -41,8 +41,10 @@ collective on the data path; value = total env-steps / max time.
 from __future__ import annotations
 
 import argparse
+import hashlib
 import json
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -96,19 +98,33 @@ def _measured_peaks() -> dict:
     return {"hbm_gbs": 6650.0, "source": "fallback"}
 
 
-def _profile_value(key: str, name: str = "control_step_contact_tree29.md") -> float | None:
-    """A `key: value` figure of a committed ncu summary under profiles/."""
+# Sources of the FP32 temporalCone control-step kernel.
+KERNEL_SOURCES = ("world_step.cu", "world_step.cuh", "contact.cuh", "dmath.cuh", "layout.h", "device_model.h")
 
-    path = ROOT / "profiles" / name
+
+def _kernel_fingerprint(folder: Path | None = None) -> str:
+    """Of KERNEL_SOURCES without comments and white space."""
+
+    digest = hashlib.sha256()
+    for name in KERNEL_SOURCES:
+        text = ((folder or ROOT / "numi_lab_b200" / "csrc") / name).read_text()
+        digest.update("".join(re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S).split()).encode())
+    return digest.hexdigest()[:16]
+
+
+def _profile_value(key: str, path: Path = ROOT / "profiles" / "control_step_contact_tree29.md") -> float | None:
+    """A `key: value` figure of a committed ncu summary; None unless it was
+    counted on the kernel that runs (`kernel_sources` names the fingerprint)."""
+
     if not path.is_file():
         return None
-    for line in path.read_text().splitlines():
-        if line.strip().startswith(key + ":"):
-            try:
-                return float(line.split(":", 1)[1].strip())
-            except ValueError:
-                return None
-    return None
+    figures = dict(line.strip().split(": ", 1) for line in path.read_text().splitlines() if ": " in line)
+    if figures.get("kernel_sources") != _kernel_fingerprint():
+        return None
+    try:
+        return float(figures[key])
+    except (KeyError, ValueError):
+        return None
 
 
 def _issue_peak() -> dict:

@@ -1671,15 +1671,17 @@ __device__ __forceinline__ void store_lambda(float* R, int c, float3 l) {
 // the same body with any number of warps, and no arithmetic depends on that
 // number, so a world's results are the same bits from either.
 //
-// What bounds it: instruction issue (47 % of cycles with one warp per
-// environment at 16 warps per SM, 13 of 32 lanes active) and, before the
-// loops were rolled, instruction fetch -- the 260 KB of an unrolled kernel
-// do not stay in the instruction cache with every warp at its own stage, and
-// the same launches ran 1.3 to 1.5 times longer.  Hence `unroll 1` on every
-// loop whose body is more than a few instructions.  Contact rows in
-// registers, arms and impulses in shared memory and the CTA per environment
-// took 16,384 36-body piles from 9.58 to 6.41 ms per control step against
-// one warp per environment with its records in global memory.
+// What bounds it: latency.  4096 settled 36-body piles at two warps per
+// environment (ncu: 14.6 warps per SM, 30 % of issue slots, 19 of 32 lanes
+// active) wait for manifold tables in L2 and HBM, for the CTA's barriers and
+// for instructions, in this order.  Before the loops were rolled it was
+// instruction fetch -- the 260 KB of an unrolled kernel do not stay in the
+// instruction cache with every warp at its own stage, and the same launches
+// ran 1.3 to 1.5 times longer.  Hence `unroll 1` on every loop whose body is
+// more than a few instructions.  Contact rows in registers, arms and impulses
+// in shared memory and the CTA per environment took 16,384 36-body piles from
+// 9.58 to 6.41 ms per control step against one warp per environment with its
+// records in global memory.
 template <bool kComp, bool kConvex>
 __device__ __noinline__ void scene_step_item(const SceneParams& p, float* s, int item, int env) {
     const int tid = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
